@@ -29,6 +29,7 @@ using mspai::Problem;
 constexpr int kBuckets = 3;    // size buckets of the planning kernel
 constexpr int kKernels = 4;    // solver launches per setup (timed separately)
 constexpr int kLists = 4;      // work lists: buckets + the overflow lists
+constexpr int kSparseLists = 3; // ... two lists between the sparse solvers' launches, small columns
 // Arena of the fixed-pattern solver's second launch (one CTA per SM): the
 // largest dynamic shared memory a CTA may have beside the solver's static part.
 constexpr int kFixedArenaLarge = 212 * 1024;
@@ -36,6 +37,20 @@ constexpr int kFixedArenaLarge = 212 * 1024;
 // updates) is at most this in FP64 directly: the FP32 QR saves nothing on such
 // sizes, and the refinement would add two passes over the column's entries.
 constexpr int kMixedFp64MaxN = 32;
+// Launches of the solvers on the sparse normal equations (fixed_cg.cu) over the
+// fixed-pattern bucket: shared memory of a column's CTA (25 KB: eight CTAs per
+// SM, 42 KB: five, 104 KB: two).  A column that does not fit goes on to the next.
+struct SparseClass {
+    int slot_bytes;
+    mspai::SparseLaunch kind;
+};
+constexpr SparseClass kSparseClasses[] = {{25 * 1024, mspai::SparseLaunch::kNarrow},
+                                          {42 * 1024, mspai::SparseLaunch::kMiddle},
+                                          {104 * 1024, mspai::SparseLaunch::kWide}};
+// Small columns: a warp each, 16 per SM (register bound).
+constexpr int kSparseTinySlot = 13 * 1024;
+constexpr int kSparseTinyN = 36;
+constexpr int kSparseTinyE = 640;
 
 // A device buffer that grows on demand.
 struct DevBuf {
@@ -124,6 +139,7 @@ struct mspai_handle {
     int warp_nmax_adaptive = 32;
     bool used_fixed = false;         // the last setup ran the fixed-pattern solver
     int64_t list_len[kLists] = {};   // columns listed per work list in the last setup
+    int64_t tiny_len = 0;            // ... and in the sparse solvers' list of small columns
 };
 
 static int set_err(mspai_handle* h, int code, const char* fmt, ...)
@@ -615,7 +631,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
     // ---- plan and bucket
     CUDA_TRY(h, h->E.ensure(sizeof(int32_t) * std::max(nprob, 1)));
     CUDA_TRY(h, h->nk.ensure(sizeof(int32_t) * std::max(nprob, 1)));
-    CUDA_TRY(h, h->lists.ensure(sizeof(int32_t) * static_cast<size_t>(kLists) *
+    CUDA_TRY(h, h->lists.ensure(sizeof(int32_t) * static_cast<size_t>(kLists + kSparseLists) *
                                 std::max(nprob, 1)));
     h->launches++;
     CUDA_TRY(h, mspai::launch_plan(pb.cptr, pb.pptr, pb.pidx, nprob, bs, h->E.as<int32_t>(),
@@ -658,6 +674,13 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
     // fixed-pattern solver (bucket 1), which sizes its arrays per column
     const bool use_fixed = !adaptive && bs == 1 && prm->batched && !pb.qru;
     rule.smem_w_bytes = use_fixed ? (int64_t(1) << 62) : h->w_smem_bytes;
+    // small fixed columns: a list of their own for the sparse solvers
+    const bool sparse = use_fixed && !out.rstore && C->nnz < (int64_t(1) << 32) &&
+                        (elem == 8 || pb.refine > 0) &&
+                        kSparseClasses[0].slot_bytes <= h->fixed_arena;
+    rule.tiny_list = sparse ? kLists + 2 : 0;
+    rule.tiny_nmax = kSparseTinyN;
+    rule.tiny_emax = kSparseTinyE;
     rule.elem_bytes = elem;
     rule.grow_n = grow_n * bs;
     rule.grow_e = adaptive ? grow_n * bs * max_col_nnz : 0;
@@ -697,10 +720,16 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
         (void)b;
         return MSPAI_OK;
     };
+    const int tiny = sparse ? hc[3] : 0;  // small columns of the sparse solvers
+    h->tiny_len = tiny;
+    if (tiny > 0) {  // their sizes belong to the fixed-pattern bucket
+        hc[4 + 1] = std::max(hc[4 + 1], hc[4 + 3]);
+        hc[8 + 1] = std::max(hc[8 + 1], hc[8 + 3]);
+    }
     for (int b = 0; b < kBuckets; b++) {
-        const int count = hc[b];
+        const int count = hc[b] + (b == 1 ? tiny : 0);
         if (!(use_fixed && b == 2))  // with the fixed-pattern solver list 2 is its overflow
-            h->list_len[b] = count;
+            h->list_len[b] = hc[b];
         if (count == 0)
             continue;
         Caps cap{};
@@ -772,8 +801,43 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
                                           mspai::fixed_max_grid(h->fixed_arena_large));
             CUDA_TRY(h, h->rglob.ensure(static_cast<size_t>(grid_max) * relems * elem));
             CUDA_TRY(h, cudaEventRecord(h->evb[2], st));
+            // the sparse normal equations first (no factor to keep; the slots
+            // count against the first launch's arena), the rest to the dense
+            // factorizations
+            const int32_t* flist = list;
+            const int32_t* fcount = nullptr;
+            if (sparse) {
+                int32_t* sc = dcnt + 28;  // rest counts [4], then queue counters [4]
+                CUDA_TRY(h, cudaMemsetAsync(sc, 0, 8 * sizeof(int32_t), st));
+                int32_t* rest = h->lists.as<int32_t>() + static_cast<size_t>(kLists) * nprob;
+                int k = 0;
+                for (const SparseClass& c : kSparseClasses) {
+                    if (c.slot_bytes > h->fixed_arena || hc[1] == 0)
+                        break;
+                    rest = h->lists.as<int32_t>() + static_cast<size_t>(kLists + k % 2) * nprob;
+                    h->launches++;
+                    CUDA_TRY(h, mspai::launch_sparse_solve(elem, c.kind, c.slot_bytes, pb, out,
+                                                           flist, fcount, hc[1], sc + 4 + k, rest,
+                                                           sc + k, st));
+                    flist = rest;
+                    fcount = sc + k;
+                    k++;
+                }
+                if (tiny > 0) {
+                    // what the small columns leave joins the rest
+                    const int32_t* tl =
+                        h->lists.as<int32_t>() + static_cast<size_t>(rule.tiny_list) * nprob;
+                    int32_t* rc3 = sc + std::max(k - 1, 0);
+                    h->launches++;
+                    CUDA_TRY(h, mspai::launch_sparse_solve(8, mspai::SparseLaunch::kTiny,
+                                                           kSparseTinySlot, pb, out, tl, nullptr,
+                                                           tiny, sc + 7, rest, rc3, st));
+                    flist = rest;
+                    fcount = rc3;
+                }
+            }
             h->launches++;
-            CUDA_TRY(h, mspai::launch_fixed_solve(elem, h->fixed_arena, pb, out, list, nullptr,
+            CUDA_TRY(h, mspai::launch_fixed_solve(elem, h->fixed_arena, pb, out, flist, fcount,
                                                   count, counter, ovf_a, cnt, h->rglob.p, relems,
                                                   grid_max, st, &grid));
             CUDA_TRY(h, cudaEventRecord(h->evb[3], st));
@@ -1091,13 +1155,16 @@ int mspai_get_stats(mspai_handle* h, mspai_stats* s)
     for (int b = 0; b < 4; b++)
         h->stats.bucket_flops[b] = 0.0;
     if (h->nprob > 0 && h->lists.p) {
-        std::vector<int32_t> lists(static_cast<size_t>(kLists) * h->nprob);
+        std::vector<int32_t> lists(static_cast<size_t>(kLists + kSparseLists) * h->nprob);
         CUDA_TRY(h, cudaMemcpy(lists.data(), h->lists.p, sizeof(int32_t) * lists.size(),
                                cudaMemcpyDeviceToHost));
         double sums[kLists] = {0.0, 0.0, 0.0, 0.0};
         for (int b = 0; b < kLists; b++)
             for (int64_t t = 0; t < h->list_len[b]; t++)
                 sums[b] += work[3 * static_cast<size_t>(lists[b * static_cast<size_t>(h->nprob) + t])];
+        for (int64_t t = 0; t < h->tiny_len; t++)
+            sums[1] += work[3 * static_cast<size_t>(
+                                lists[(kLists + 2) * static_cast<size_t>(h->nprob) + t])];
         if (h->used_fixed) {
             h->stats.bucket_flops[0] = sums[0];
             h->stats.bucket_flops[1] = sums[1] - sums[2];

@@ -59,7 +59,8 @@ __global__ void plan_kernel(const int64_t* __restrict__ cptr, const int64_t* __r
     }
 }
 
-// bucket ids: 0 warp (tiny), 1 CTA + shared-memory W, 2 CTA + global W
+// bucket ids: 0 warp (tiny), 1 CTA + shared-memory W, 2 CTA + global W,
+// 3 small columns of the sparse solver
 __global__ void bucket_kernel(const int32_t* __restrict__ E, const int32_t* __restrict__ nk, int n,
                               BucketRule rule, int32_t* __restrict__ counts,
                               int32_t* __restrict__ maxE, int32_t* __restrict__ maxN,
@@ -79,13 +80,15 @@ __global__ void bucket_kernel(const int32_t* __restrict__ E, const int32_t* __re
             b = rule.single_bucket;
         else if (rule.allow_warp && ef <= rule.warp_emax && nf <= rule.warp_nmax)
             b = 0;
+        else if (rule.tiny_list > 0 && ef <= rule.tiny_emax && nf <= rule.tiny_nmax)
+            b = 3;
         else {
             const int64_t mw = ef / 2 + nf;
             const int64_t wbytes = (mw * nf + mw) * rule.elem_bytes;
             b = (wbytes <= rule.smem_w_bytes) ? 1 : 2;
         }
         const int slot = atomicAdd(&counts[b], 1);
-        lists[static_cast<int64_t>(b) * n + slot] = col;
+        lists[static_cast<int64_t>(b == 3 ? rule.tiny_list : b) * n + slot] = col;
         atomicMax(&maxE[b], static_cast<int32_t>(ef > 0x7fffffff ? 0x7fffffff : ef));
         atomicMax(&maxN[b], static_cast<int32_t>(nf));
     }

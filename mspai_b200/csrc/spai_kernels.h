@@ -25,6 +25,9 @@ struct BucketRule {
     int grow_e;            // mn * ns * max column nnz of C
     const int32_t* rep;    // reuse table: columns with rep[k] != k are skipped (nullable)
     int lo, hi;            // only problem columns [lo, hi) are binned
+    int tiny_list;         // > 0: work list of bucket 3, small columns of the sparse
+    int tiny_nmax;         // solver: |J| and
+    int tiny_emax;         // entries of C(:,J) at most these
 };
 
 // Row structure (CSR) of a CSC matrix, in ascending column order within each
@@ -90,6 +93,19 @@ cudaError_t launch_fixed_solve(int elem_bytes, int arena_bytes, const Problem& p
                                int count_host, int32_t* counter, int32_t* ovf_list,
                                int32_t* ovf_count, void* rglob, int64_t rglob_elems, int max_ctas,
                                cudaStream_t st, int* grid_out);
+// Solvers on the sparse normal equations (fixed_cg.cu), a CTA per column in
+// slot_bytes of shared memory; the columns that one does not take go to
+// ovf_list / *ovf_count (appended).  nnz(C) < 2^32.
+enum class SparseLaunch {
+    kTiny,    // a warp per column, |J| <= 36, FP64
+    kNarrow,  // four warps, |J| <= 144
+    kMiddle,  // four warps, |J| <= 272
+    kWide     // four warps, |J| <= 400
+};
+cudaError_t launch_sparse_solve(int elem_bytes, SparseLaunch kind, int slot_bytes,
+                                const Problem& pb, const Output& out, const int32_t* list,
+                                const int32_t* count_dev, int count_host, int32_t* counter,
+                                int32_t* ovf_list, int32_t* ovf_count, cudaStream_t st);
 cudaError_t launch_scan_lengths(const int32_t* len, int n, int64_t* ptr, int64_t* tmp,
                                 cudaStream_t st);
 // len[k] = |P(:, k)| (|P(:, k)| + 1) / 2 (packed triangles of the kept R)
