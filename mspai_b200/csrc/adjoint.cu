@@ -245,25 +245,30 @@ __device__ void adjoint_column(const G& g, const Problem& pb, const Caps& cap, S
 }
 
 // E[k] = entries of C(:, J_k), nk[k] = |J_k| for problem column k, J_k the
-// pattern of scalar column bs k of the result
+// pattern of scalar column bs k of the result; eight lanes per column
 __global__ void adjoint_plan_kernel(const int64_t* __restrict__ cptr,
                                     const int64_t* __restrict__ mptr,
                                     const int32_t* __restrict__ midx, int nprob, int bs,
                                     int32_t* __restrict__ E, int32_t* __restrict__ nk)
 {
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int kb = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; kb < nprob; kb += warps) {
-        const int64_t a = mptr[bs * kb], b = mptr[bs * kb + 1];
-        int64_t e = 0;
-        for (int64_t p = a + lane; p < b; p += 32) {
+    const int lane = threadIdx.x & 7;
+    const int groups = (gridDim.x * blockDim.x) >> 3;
+    const int first = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    for (int64_t base = 0; base < nprob; base += groups) {  // every lane of a warp takes part
+        const int64_t kb = base + first;
+        int64_t a = 0, b = 0, e = 0;
+        if (kb < nprob) {
+            a = mptr[bs * kb];
+            b = mptr[bs * kb + 1];
+        }
+        for (int64_t p = a + lane; p < b; p += 8) {
             const int j = midx[p];
             e += cptr[j + 1] - cptr[j];
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+        for (int o = 4; o > 0; o >>= 1)
             e += __shfl_xor_sync(0xffffffffu, e, o);
-        if (lane == 0) {
+        if (lane == 0 && kb < nprob) {
             E[kb] = static_cast<int32_t>(e > 0x7fffffff ? 0x7fffffff : e);
             nk[kb] = static_cast<int32_t>(b - a);
         }
@@ -275,15 +280,15 @@ cudaError_t launch_adjoint_plan(const int64_t* cptr, const int64_t* mptr, const 
 {
     if (nprob <= 0)
         return cudaSuccess;
-    const int blocks = std::max(1, std::min((nprob + 7) / 8, num_sms() * 16));
+    const int blocks = std::max(1, std::min((nprob + 31) / 32, num_sms() * 8));
     adjoint_plan_kernel<<<blocks, 256, 0, st>>>(cptr, mptr, midx, nprob, bs, E, nk);
     return cudaGetLastError();
 }
 
 template <class TR, int NT>
 __global__ void __launch_bounds__(NT)
-    adjoint_cta_kernel(Problem pb, Caps cap, AdjointIO io, int lo, int hi, char* scratch,
-                       size_t slot_bytes, int32_t* counter)
+    adjoint_cta_kernel(Problem pb, Caps cap, AdjointIO io, const int32_t* __restrict__ list,
+                       int count, char* scratch, size_t slot_bytes, int32_t* counter)
 {
     __shared__ GroupScratch sc;
     CtaGroup<NT> g{&sc};
@@ -291,20 +296,20 @@ __global__ void __launch_bounds__(NT)
     Slot<double> s = lay.at(scratch + static_cast<size_t>(blockIdx.x) * slot_bytes, nullptr);
     while (true) {
         if (threadIdx.x == 0)
-            sc.i[5] = lo + atomicAdd(counter, 1);
+            sc.i[5] = atomicAdd(counter, 1);
         __syncthreads();
-        const int col = sc.i[5];
+        const int t = sc.i[5];
         __syncthreads();
-        if (col >= hi)
+        if (t >= count)
             break;
-        adjoint_column<TR>(g, pb, cap, s, io, col);
+        adjoint_column<TR>(g, pb, cap, s, io, list[t]);
     }
 }
 
 template <class TR>
 __global__ void __launch_bounds__(kWarpKernelThreads)
-    adjoint_warp_kernel(Problem pb, Caps cap, AdjointIO io, int lo, int hi, char* scratch,
-                        size_t slot_bytes, int32_t* counter)
+    adjoint_warp_kernel(Problem pb, Caps cap, AdjointIO io, const int32_t* __restrict__ list,
+                        int count, char* scratch, size_t slot_bytes, int32_t* counter)
 {
     __shared__ GroupScratch sc[kWarpKernelThreads / 32];
     const int w = threadIdx.x >> 5;
@@ -314,47 +319,219 @@ __global__ void __launch_bounds__(kWarpKernelThreads)
     const size_t slot_id = static_cast<size_t>(blockIdx.x) * (kWarpKernelThreads / 32) + w;
     Slot<double> s = lay.at(scratch + slot_id * slot_bytes, nullptr);
     while (true) {
-        int col = 0;
+        int t = 0;
         if (lane == 0)
-            col = lo + atomicAdd(counter, 1);
-        col = __shfl_sync(0xffffffffu, col, 0);
-        if (col >= hi)
+            t = atomicAdd(counter, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >= count)
             break;
-        adjoint_column<TR>(g, pb, cap, s, io, col);
+        adjoint_column<TR>(g, pb, cap, s, io, list[t]);
     }
 }
 
 template <class TR>
-static void launch_adjoint_t(const Problem& pb, const Caps& cap, const AdjointIO& io, int lo,
-                             int hi, bool warp, char* scratch, size_t scratch_bytes,
-                             int32_t* counter, cudaStream_t st)
+static void launch_adjoint_t(const Problem& pb, const Caps& cap, const AdjointIO& io,
+                             const int32_t* list, int n, bool warp, char* scratch,
+                             size_t scratch_bytes, int32_t* counter, cudaStream_t st)
 {
-    const int n = hi - lo;  // columns of this launch
     const size_t slot = SlotLayout<double>(cap, false).bytes;
     const int sms = num_sms();
     if (warp) {
         const int per_block = kWarpKernelThreads / 32;
         int grid = std::min<int>(sms * 8, (n + per_block - 1) / per_block);
         grid = std::max(1, std::min<int>(grid, static_cast<int>(scratch_bytes / (slot * per_block))));
-        adjoint_warp_kernel<TR><<<grid, kWarpKernelThreads, 0, st>>>(pb, cap, io, lo, hi, scratch,
+        adjoint_warp_kernel<TR><<<grid, kWarpKernelThreads, 0, st>>>(pb, cap, io, list, n, scratch,
                                                                      slot, counter);
     }
     else {
         int grid = std::min(sms * 4, n);
         grid = std::max(1, std::min<int>(grid, static_cast<int>(scratch_bytes / slot)));
-        adjoint_cta_kernel<TR, 128><<<grid, 128, 0, st>>>(pb, cap, io, lo, hi, scratch, slot,
+        adjoint_cta_kernel<TR, 128><<<grid, 128, 0, st>>>(pb, cap, io, list, n, scratch, slot,
                                                           counter);
     }
 }
 
-cudaError_t launch_adjoint(const Problem& pb, const Caps& cap, const AdjointIO& io, int lo,
-                           int hi, bool warp, char* scratch, size_t scratch_bytes,
-                           int32_t* counter, cudaStream_t st)
+cudaError_t launch_adjoint(const Problem& pb, const Caps& cap, const AdjointIO& io,
+                           const int32_t* list, int count, bool warp, char* scratch,
+                           size_t scratch_bytes, int32_t* counter, cudaStream_t st)
 {
     if (io.rstore && io.r_elem == 4)
-        launch_adjoint_t<float>(pb, cap, io, lo, hi, warp, scratch, scratch_bytes, counter, st);
+        launch_adjoint_t<float>(pb, cap, io, list, count, warp, scratch, scratch_bytes, counter,
+                                st);
     else
-        launch_adjoint_t<double>(pb, cap, io, lo, hi, warp, scratch, scratch_bytes, counter, st);
+        launch_adjoint_t<double>(pb, cap, io, list, count, warp, scratch, scratch_bytes, counter,
+                                 st);
+    return cudaGetLastError();
+}
+
+// Scalar columns of at most eight unknowns without a gbar, eight lanes per
+// column, four columns per warp.  Lane j walks the sorted entries of C(:, J(j));
+// the smallest head of the eight lanes is the next row of I_k, its residual is
+// the target's value there less the sum of the lanes' products, and the lanes
+// with an entry in the row add -2 w r x_j to dC.  Nothing is stored or sorted.
+// Bound: the FP64 atomics on dC and the latency of the reads of C (1,048,576
+// columns of 35 entries: 6.8 ms in the warp kernel above, 0.54 ms here).
+__global__ void __launch_bounds__(256)
+    adjoint_small_kernel(Problem pb, AdjointIO io, const int32_t* __restrict__ list, int count)
+{
+    constexpr uint32_t all = 0xffffffffu;
+    const int lane = threadIdx.x & 31, grp = lane >> 3, l8 = lane & 7;
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    for (int64_t t0 = 4 * static_cast<int64_t>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+         t0 < count; t0 += 4 * static_cast<int64_t>(warps)) {
+        const int col = t0 + grp < count ? list[t0 + grp] : -1;
+        int64_t e = 0, e1 = 0, q = 0, q1 = 0;
+        double x = 0.0;
+        if (col >= 0) {
+            const int64_t p0 = io.mptr[col];
+            const int n = static_cast<int>(io.mptr[col + 1] - p0);
+            if (l8 < n) {
+                const int j = io.midx[p0 + l8];
+                x = io.mval[p0 + l8];
+                e = pb.cptr[j];
+                e1 = pb.cptr[j + 1];
+            }
+            if (pb.bptr) {
+                q = pb.bptr[col];
+                q1 = pb.bptr[col + 1];
+            }
+        }
+        int row = e < e1 ? __ldg(pb.cidx + e) : 0x7fffffff;
+        double val = e < e1 ? __ldg(pb.cval + e) : 0.0;
+        int brow = q < q1 ? __ldg(pb.bidx + q) : 0x7fffffff;
+        double loss = 0.0;
+        bool seen = pb.bptr != nullptr || col < 0;  // identity target: e_col met in I_k
+        // target entries in rows outside I_k, up to row `below`
+        auto outside = [&](int below) {
+            while (brow < below) {
+                const double b = pb.bval[q];
+                loss += b * b;
+                if (io.dB && l8 == 0)
+                    io.dB[q] = 2.0 * io.wres * b;
+                q++;
+                brow = q < q1 ? __ldg(pb.bidx + q) : 0x7fffffff;
+            }
+        };
+        while (true) {
+            int low = min(row, __shfl_xor_sync(all, row, 4));
+            low = min(low, __shfl_xor_sync(all, low, 2));
+            low = min(low, __shfl_xor_sync(all, low, 1));
+            const bool more = low != 0x7fffffff;
+            if (!__any_sync(all, more))
+                break;
+            const bool mine = more && row == low;
+            double s = mine ? val * x : 0.0;
+            s += __shfl_xor_sync(all, s, 4);
+            s += __shfl_xor_sync(all, s, 2);
+            s += __shfl_xor_sync(all, s, 1);
+            if (!more)
+                continue;
+            double b = 0.0;
+            outside(low);
+            const bool hit = brow == low;
+            if (hit)
+                b = pb.bval[q];
+            else if (pb.bptr == nullptr && low == col) {
+                b = 1.0;
+                seen = true;
+            }
+            const double r = b - s;
+            loss += r * r;
+            if (hit) {
+                if (io.dB && l8 == 0)
+                    io.dB[q] = 2.0 * io.wres * r;
+                q++;
+                brow = q < q1 ? __ldg(pb.bidx + q) : 0x7fffffff;
+            }
+            if (mine) {
+                atomicAdd(&io.dC[e], -(r * x) * (2.0 * io.wres));
+                e++;
+                row = e < e1 ? __ldg(pb.cidx + e) : 0x7fffffff;
+                val = e < e1 ? __ldg(pb.cval + e) : 0.0;
+            }
+        }
+        outside(0x7fffffff);
+        if (!seen)
+            loss += 1.0;  // e_col has its 1 outside I_k
+        if (l8 == 0 && col >= 0)
+            io.loss[col] = io.wres * loss;
+        __syncwarp();
+    }
+}
+
+cudaError_t launch_adjoint_small(const Problem& pb, const AdjointIO& io, const int32_t* list,
+                                 int count, cudaStream_t st)
+{
+    if (count <= 0)
+        return cudaSuccess;
+    const int blocks = std::max(1, std::min((count + 31) / 32, num_sms() * 8));
+    adjoint_small_kernel<<<blocks, 256, 0, st>>>(pb, io, list, count);
+    return cudaGetLastError();
+}
+
+// s + c += v, exactly up to the last bits of c (Neumaier).
+__device__ __forceinline__ void add_compensated(double& s, double& c, double v)
+{
+    const double t = s + v;
+    c += fabs(s) >= fabs(v) ? (s - t) + v : (v - t) + s;
+    s = t;
+}
+
+// The columns' losses are often nearly equal and a plain sum of a million lets
+// their rounding errors add up: every thread sums its share with compensation,
+// and the pairs are combined in a fixed order.  (On the host this took 3 ms a
+// call for 1,048,576 columns, the copy included.)
+__global__ void __launch_bounds__(256)
+    loss_parts_kernel(const double* __restrict__ v, int n, double* __restrict__ parts)
+{
+    __shared__ double ss[256], sc[256];
+    double s = 0.0, c = 0.0;
+    for (int64_t i = blockIdx.x * 256 + threadIdx.x; i < n; i += 256 * static_cast<int64_t>(gridDim.x))
+        add_compensated(s, c, v[i]);
+    ss[threadIdx.x] = s;
+    sc[threadIdx.x] = c;
+    for (int o = 128; o > 0; o >>= 1) {
+        __syncthreads();
+        if (threadIdx.x < o) {
+            double a = ss[threadIdx.x], b = sc[threadIdx.x];
+            add_compensated(a, b, ss[threadIdx.x + o]);
+            b += sc[threadIdx.x + o];
+            ss[threadIdx.x] = a;
+            sc[threadIdx.x] = b;
+        }
+    }
+    if (threadIdx.x == 0) {
+        parts[2 * blockIdx.x] = ss[0];
+        parts[2 * blockIdx.x + 1] = sc[0];
+    }
+}
+
+__global__ void loss_total_kernel(const double* __restrict__ parts, int n, double* __restrict__ total)
+{
+    __shared__ double ss[kLossParts], sc[kLossParts];
+    for (int i = threadIdx.x; i < kLossParts; i += blockDim.x) {
+        ss[i] = i < n ? parts[2 * i] : 0.0;
+        sc[i] = i < n ? parts[2 * i + 1] : 0.0;
+    }
+    for (int o = kLossParts / 2; o > 0; o >>= 1) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < o; i += blockDim.x) {
+            double a = ss[i], b = sc[i];
+            add_compensated(a, b, ss[i + o]);
+            b += sc[i + o];
+            ss[i] = a;
+            sc[i] = b;
+        }
+    }
+    if (threadIdx.x == 0)
+        *total = ss[0] + sc[0];
+}
+
+cudaError_t launch_loss_sum(const double* v, int n, double* tmp, double* total, cudaStream_t st)
+{
+    const int blocks = std::max(1, std::min((n + 1023) / 1024, kLossParts));
+    loss_parts_kernel<<<blocks, 256, 0, st>>>(v, n, tmp);
+    loss_total_kernel<<<1, 256, 0, st>>>(tmp, blocks, total);
     return cudaGetLastError();
 }
 

@@ -29,7 +29,8 @@ using mspai::Problem;
 constexpr int kBuckets = 3;    // size buckets of the planning kernel
 constexpr int kKernels = 4;    // solver launches per setup (timed separately)
 constexpr int kLists = 4;      // work lists: buckets + the overflow lists
-constexpr int kSparseLists = 3; // ... two lists between the sparse solvers' launches, small columns
+constexpr int kMoreLists = 5;  // ... two between the sparse solvers' launches, their small
+                               // columns, the small QR's columns and its tall ones
 // Arena of the fixed-pattern solver's second launch (one CTA per SM): the
 // largest dynamic shared memory a CTA may have beside the solver's static part.
 constexpr int kFixedArenaLarge = 212 * 1024;
@@ -105,6 +106,7 @@ struct mspai_handle {
     DevBuf scratch;
     DevBuf vflag;  // device input checks
     DevBuf ax, ay; // host vectors of mspai_apply
+    DevBuf aloss, acnt;  // losses and counters of the adjoint
     // row structure of the result for mspai_apply (built on first use)
     DevBuf tptr, tcol, tval, tkeys, tperm0, tperm1, tcnt, ttemp;
     bool rows_valid = false;
@@ -139,7 +141,8 @@ struct mspai_handle {
     int warp_nmax_adaptive = 32;
     bool used_fixed = false;         // the last setup ran the fixed-pattern solver
     int64_t list_len[kLists] = {};   // columns listed per work list in the last setup
-    int64_t tiny_len = 0;            // ... and in the sparse solvers' list of small columns
+    int64_t tiny_len = 0;            // ... in the sparse solvers' list of small columns
+    int64_t small_len = 0;           // ... and in the small QR's
 };
 
 static int set_err(mspai_handle* h, int code, const char* fmt, ...)
@@ -277,7 +280,7 @@ void mspai_free(mspai_handle* h)
                       &h->midx, &h->mval, &h->scratch, &h->vflag, &h->ax, &h->ay,
                       &h->rkeys, &h->rslot_rep, &h->rslot_of, &h->rrep, &h->tptr, &h->tcol,
                       &h->tval, &h->tkeys, &h->tperm0, &h->tperm1, &h->tcnt, &h->ttemp,
-                      &h->rglob};
+                      &h->rglob, &h->aloss, &h->acnt};
     for (DevBuf* b : bufs)
         b->release();
     if (h->ev0)
@@ -631,7 +634,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
     // ---- plan and bucket
     CUDA_TRY(h, h->E.ensure(sizeof(int32_t) * std::max(nprob, 1)));
     CUDA_TRY(h, h->nk.ensure(sizeof(int32_t) * std::max(nprob, 1)));
-    CUDA_TRY(h, h->lists.ensure(sizeof(int32_t) * static_cast<size_t>(kLists + kSparseLists) *
+    CUDA_TRY(h, h->lists.ensure(sizeof(int32_t) * static_cast<size_t>(kLists + kMoreLists) *
                                 std::max(nprob, 1)));
     h->launches++;
     CUDA_TRY(h, mspai::launch_plan(pb.cptr, pb.pptr, pb.pidx, nprob, bs, h->E.as<int32_t>(),
@@ -674,6 +677,10 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
     // fixed-pattern solver (bucket 1), which sizes its arrays per column
     const bool use_fixed = !adaptive && bs == 1 && prm->batched && !pb.qru;
     rule.smem_w_bytes = use_fixed ? (int64_t(1) << 62) : h->w_smem_bytes;
+    // the smallest fixed columns: eight lanes each (the store of R holds one
+    // element type, the small QR is FP64: not when R is kept)
+    const bool small = use_fixed && !out.rstore;
+    rule.small_list = small ? kLists + 3 : 0;
     // small fixed columns: a list of their own for the sparse solvers
     const bool sparse = use_fixed && !out.rstore && C->nnz < (int64_t(1) << 32) &&
                         (elem == 8 || pb.refine > 0) &&
@@ -720,6 +727,23 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
         (void)b;
         return MSPAI_OK;
     };
+    const int nsmall = small ? hc[2] : 0;
+    if (small)
+        hc[2] = 0;
+    if (nsmall > 0) {
+        int32_t* lists = h->lists.as<int32_t>();
+        int32_t* rc = dcnt + 36;
+        CUDA_TRY(h, cudaMemsetAsync(rc, 0, 2 * sizeof(int32_t), st));
+        CUDA_TRY(h, cudaEventRecord(h->evb[0], st));
+        h->launches += 2;
+        CUDA_TRY(h, mspai::launch_small_qr(
+                        pb, out, lists + static_cast<size_t>(kLists + 3) * nprob, nsmall,
+                        lists + static_cast<size_t>(kLists + 4) * nprob, rc, st));
+        CUDA_TRY(h, cudaEventRecord(h->evb[1], st));
+        timed[0] = true;
+        h->stats.bucket_columns[0] = nsmall;
+    }
+    h->small_len = nsmall;
     const int tiny = sparse ? hc[3] : 0;  // small columns of the sparse solvers
     h->tiny_len = tiny;
     if (tiny > 0) {  // their sizes belong to the fixed-pattern bucket
@@ -770,23 +794,25 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             CUDA_TRY(h, h->scratch.ensure(need));
             if (adaptive)  // the candidate bit vectors of the slots start cleared
                 CUDA_TRY(h, cudaMemsetAsync(h->scratch.p, 0, need, st));
-            CUDA_TRY(h, cudaEventRecord(h->evb[0], st));
+            if (nsmall == 0)
+                CUDA_TRY(h, cudaEventRecord(h->evb[0], st));
             h->launches++;
             CUDA_TRY(h, mspai::launch_warp_solve_global(elem_b, pbb, cap, out, list, count,
                                                         counter, h->scratch.as<char>(),
                                                         h->scratch.bytes, st, &grid));
             CUDA_TRY(h, cudaEventRecord(h->evb[1], st));
             timed[0] = true;
-            h->stats.bucket_columns[0] = count;
+            h->stats.bucket_columns[0] = count + nsmall;
         }
         else if (use_warp) {
-            CUDA_TRY(h, cudaEventRecord(h->evb[0], st));
+            if (nsmall == 0)
+                CUDA_TRY(h, cudaEventRecord(h->evb[0], st));
             h->launches++;
             CUDA_TRY(h, mspai::launch_warp_solve(elem_b, pbb, cap, out, list, count, counter, st,
                                                  &grid));
             CUDA_TRY(h, cudaEventRecord(h->evb[1], st));
             timed[0] = true;
-            h->stats.bucket_columns[0] = count;
+            h->stats.bucket_columns[0] = count + nsmall;
         }
         else if (b == 1 && use_fixed) {
             // fixed-pattern solver: launch A (tuned arena) over the bucket, its
@@ -1155,7 +1181,7 @@ int mspai_get_stats(mspai_handle* h, mspai_stats* s)
     for (int b = 0; b < 4; b++)
         h->stats.bucket_flops[b] = 0.0;
     if (h->nprob > 0 && h->lists.p) {
-        std::vector<int32_t> lists(static_cast<size_t>(kLists + kSparseLists) * h->nprob);
+        std::vector<int32_t> lists(static_cast<size_t>(kLists + kMoreLists) * h->nprob);
         CUDA_TRY(h, cudaMemcpy(lists.data(), h->lists.p, sizeof(int32_t) * lists.size(),
                                cudaMemcpyDeviceToHost));
         double sums[kLists] = {0.0, 0.0, 0.0, 0.0};
@@ -1165,6 +1191,9 @@ int mspai_get_stats(mspai_handle* h, mspai_stats* s)
         for (int64_t t = 0; t < h->tiny_len; t++)
             sums[1] += work[3 * static_cast<size_t>(
                                 lists[(kLists + 2) * static_cast<size_t>(h->nprob) + t])];
+        for (int64_t t = 0; t < h->small_len; t++)
+            sums[0] += work[3 * static_cast<size_t>(
+                                lists[(kLists + 3) * static_cast<size_t>(h->nprob) + t])];
         if (h->used_fixed) {
             h->stats.bucket_flops[0] = sums[0];
             h->stats.bucket_flops[1] = sums[1] - sums[2];
@@ -1243,7 +1272,9 @@ extern "C" int mspai_adjoint_weighted(mspai_handle* h, const mspai_csc* C, const
     io.midx = h->res_idx;
     io.mval = h->res_val;
     io.wres = residual_weight;
-    DevBuf gbuf, dcbuf, dbbuf, lossbuf, cnt;
+    DevBuf gbuf, dcbuf, dbbuf;
+    // kept in the handle: the columns' losses with their sum, the counters
+    DevBuf &lossbuf = h->aloss, &cnt = h->acnt;
     if (gbar_values) {
         const double* gp = nullptr;
         CUDA_TRY(h, stage(gbuf, gbar_values, static_cast<size_t>(h->nnz_m), mem, st, &gp));
@@ -1269,7 +1300,7 @@ extern "C" int mspai_adjoint_weighted(mspai_handle* h, const mspai_csc* C, const
     CUDA_TRY(h, cudaMemsetAsync(io.dC, 0, sizeof(double) * C->nnz, st));
     if (io.dB)  // entries of columns outside the setup's range stay zero
         CUDA_TRY(h, cudaMemsetAsync(io.dB, 0, sizeof(double) * B->nnz, st));
-    CUDA_TRY(h, lossbuf.ensure(sizeof(double) * std::max(nprob, 1)));
+    CUDA_TRY(h, lossbuf.ensure(sizeof(double) * (std::max(nprob, 1) + 2 * mspai::kLossParts + 1)));
     io.loss = lossbuf.as<double>();
     CUDA_TRY(h, cudaMemsetAsync(io.loss, 0, sizeof(double) * std::max(nprob, 1), st));
     // sizes: entries and pattern length of each problem column at the result's pattern
@@ -1287,6 +1318,9 @@ extern "C" int mspai_adjoint_weighted(mspai_handle* h, const mspai_csc* C, const
     const int ahi = h->last_params.col_end > 0 ? h->last_params.col_end : nprob;
     BucketRule rule{};
     rule.single_bucket = 0;
+    // scalar columns of at most eight unknowns: eight lanes each (the residual
+    // term alone: gbar needs the factor)
+    rule.small_list = (bs == 1 && !gbar_values) ? 2 : 0;
     rule.elem_bytes = 8;
     rule.lo = alo;
     rule.hi = ahi;
@@ -1296,26 +1330,39 @@ extern "C" int mspai_adjoint_weighted(mspai_handle* h, const mspai_csc* C, const
     int32_t hc[16];
     CUDA_TRY(h, cudaMemcpyAsync(hc, dcnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(h, cudaStreamSynchronize(st));
-    Caps cap{};
-    cap.emax = std::max(1, hc[4]);
-    cap.nmax = std::max(1, hc[8]);
-    cap.lsort = mspai::next_pow2(cap.emax);
-    cap.mwmax = cap.emax / 2 + cap.nmax;
-    cap.cmax = cap.emax;  // q = C lambda is kept in the rho[] area
-    cap.lcand = 0;
-    cap.nrhs = bs;
-    cap.nbmap = 0;
-    const bool warp = cap.emax <= 64 && cap.nmax <= 16;
-    const size_t need = mspai::adjoint_scratch_bytes(cap, nprob, warp);
-    CUDA_TRY(h, h->scratch.ensure(need));
-    CUDA_TRY(h, cudaMemsetAsync(dcnt + 20, 0, sizeof(int32_t), st));
-    h->launches++;
-    CUDA_TRY(h, mspai::launch_adjoint(pb, cap, io, alo, ahi, warp, h->scratch.as<char>(),
-                                      h->scratch.bytes, dcnt + 20, st));
-    std::vector<double> hl(nprob);
-    if (nprob > 0)
-        CUDA_TRY(h, cudaMemcpyAsync(hl.data(), io.loss, sizeof(double) * nprob,
+    if (hc[2] > 0) {
+        h->launches++;
+        CUDA_TRY(h, mspai::launch_adjoint_small(
+                        pb, io, h->lists.as<int32_t>() + 2 * static_cast<size_t>(nprob), hc[2],
+                        st));
+    }
+    if (hc[0] > 0) {
+        Caps cap{};
+        cap.emax = std::max(1, hc[4]);
+        cap.nmax = std::max(1, hc[8]);
+        cap.lsort = mspai::next_pow2(cap.emax);
+        cap.mwmax = cap.emax / 2 + cap.nmax;
+        cap.cmax = cap.emax;  // q = C lambda is kept in the rho[] area
+        cap.lcand = 0;
+        cap.nrhs = bs;
+        cap.nbmap = 0;
+        const bool warp = cap.emax <= 64 && cap.nmax <= 16;
+        const size_t need = mspai::adjoint_scratch_bytes(cap, hc[0], warp);
+        CUDA_TRY(h, h->scratch.ensure(need));
+        CUDA_TRY(h, cudaMemsetAsync(dcnt + 20, 0, sizeof(int32_t), st));
+        h->launches++;
+        CUDA_TRY(h, mspai::launch_adjoint(pb, cap, io, h->lists.as<int32_t>(), hc[0], warp,
+                                          h->scratch.as<char>(), h->scratch.bytes, dcnt + 20,
+                                          st));
+    }
+    double total = 0.0;
+    {
+        double* tmp = io.loss + std::max(nprob, 1);
+        h->launches += 2;
+        CUDA_TRY(h, mspai::launch_loss_sum(io.loss, nprob, tmp, tmp + 2 * mspai::kLossParts, st));
+        CUDA_TRY(h, cudaMemcpyAsync(&total, tmp + 2 * mspai::kLossParts, sizeof(double),
                                     cudaMemcpyDeviceToHost, st));
+    }
     if (mem == MSPAI_MEM_HOST) {
         CUDA_TRY(h, cudaMemcpyAsync(dC_values, io.dC, sizeof(double) * C->nnz,
                                     cudaMemcpyDeviceToHost, st));
@@ -1325,21 +1372,10 @@ extern "C" int mspai_adjoint_weighted(mspai_handle* h, const mspai_csc* C, const
     }
     CUDA_TRY(h, cudaStreamSynchronize(st));
     CUDA_TRY(h, cudaGetLastError());
-    if (loss) {
-        // compensated (Neumaier) sum: the columns' losses are often nearly
-        // equal, and a plain running sum lets their rounding errors add up
-        double s = 0.0, comp = 0.0;
-        for (double v : hl) {
-            const double t = s + v;
-            comp += std::fabs(s) >= std::fabs(v) ? (s - t) + v : (v - t) + s;
-            s = t;
-        }
-        *loss = s + comp;
-    }
+    if (loss)
+        *loss = total;
     gbuf.release();
     dcbuf.release();
     dbbuf.release();
-    lossbuf.release();
-    cnt.release();
     return MSPAI_OK;
 }

@@ -35,62 +35,130 @@ extern "C" int mspai_profile_phase_cycles(unsigned long long* out, int reset)
 #endif
 
 // ------------------------------------------------------------------ planning
+// Eight lanes per column: a stencil's pattern has five to 27 entries, and a warp
+// per column left most lanes idle (1,048,576 columns of five entries: 177 us,
+// eight lanes 88 us).
 __global__ void plan_kernel(const int64_t* __restrict__ cptr, const int64_t* __restrict__ pptr,
                             const int32_t* __restrict__ pidx, int nprob, int bs,
                             int32_t* __restrict__ E, int32_t* __restrict__ nk)
 {
-    const int lane = threadIdx.x & 31;
-    const int warps = (gridDim.x * blockDim.x) >> 5;
-    for (int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; col < nprob; col += warps) {
-        const int64_t a = pptr[col], b = pptr[col + 1];
-        int64_t e = 0;
-        for (int64_t p = a + lane; p < b; p += 32) {
+    const int lane = threadIdx.x & 7;
+    const int groups = (gridDim.x * blockDim.x) >> 3;
+    const int first = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    for (int64_t base = 0; base < nprob; base += groups) {  // every lane of a warp takes part
+        const int64_t col = base + first;
+        int64_t a = 0, b = 0, e = 0;
+        if (col < nprob) {
+            a = pptr[col];
+            b = pptr[col + 1];
+        }
+        for (int64_t p = a + lane; p < b; p += 8) {
             const int j = pidx[p];
-            for (int c = 0; c < bs; c++)
-                e += cptr[bs * j + c + 1] - cptr[bs * j + c];
+            e += cptr[bs * j + bs] - cptr[bs * j];
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+        for (int o = 4; o > 0; o >>= 1)
             e += __shfl_xor_sync(0xffffffffu, e, o);
-        if (lane == 0) {
+        if (lane == 0 && col < nprob) {
             E[col] = static_cast<int32_t>(e > 0x7fffffff ? 0x7fffffff : e);
             nk[col] = static_cast<int32_t>((b - a) * bs);
         }
     }
 }
 
-// bucket ids: 0 warp (tiny), 1 CTA + shared-memory W, 2 CTA + global W,
-// 3 small columns of the sparse solver
-__global__ void bucket_kernel(const int32_t* __restrict__ E, const int32_t* __restrict__ nk, int n,
-                              BucketRule rule, int32_t* __restrict__ counts,
-                              int32_t* __restrict__ maxE, int32_t* __restrict__ maxN,
-                              int32_t* __restrict__ lists)
+// bucket ids: 0 warp (tiny), 1 CTA + shared-memory W, 2 CTA + global W (with a
+// small_list: columns of the small QR instead), 3 small columns of the sparse solver
+// A block bins kBinTile columns at a time: the places inside the tile are counted
+// in shared memory, and the tile takes its places in the lists with one atomic
+// per bucket (one atomic per column serialised on three addresses: 1.37 ms for
+// 1,048,576 columns, 18 us now).
+constexpr int kBinThreads = 256;
+constexpr int kBinTile = 4 * kBinThreads;
+
+__global__ void __launch_bounds__(kBinThreads)
+    bucket_kernel(const int32_t* __restrict__ E, const int32_t* __restrict__ nk, int n,
+                  BucketRule rule, int32_t* __restrict__ counts, int32_t* __restrict__ maxE,
+                  int32_t* __restrict__ maxN, int32_t* __restrict__ lists)
 {
-    for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < n;
-         col += gridDim.x * blockDim.x) {
-        if (col < rule.lo || col >= rule.hi)
-            continue;  // outside the requested column range
-        if (rule.rep && rule.rep[col] != col)
-            continue;  // solved by its representative
-        // sizes after at most ns pattern updates
-        const int64_t nf = static_cast<int64_t>(nk[col]) + rule.grow_n;
-        const int64_t ef = static_cast<int64_t>(E[col]) + rule.grow_e;
-        int b;
-        if (rule.single_bucket >= 0)
-            b = rule.single_bucket;
-        else if (rule.allow_warp && ef <= rule.warp_emax && nf <= rule.warp_nmax)
-            b = 0;
-        else if (rule.tiny_list > 0 && ef <= rule.tiny_emax && nf <= rule.tiny_nmax)
-            b = 3;
-        else {
-            const int64_t mw = ef / 2 + nf;
-            const int64_t wbytes = (mw * nf + mw) * rule.elem_bytes;
-            b = (wbytes <= rule.smem_w_bytes) ? 1 : 2;
+    __shared__ int32_t tile_count[4], tile_base[4];
+    const int lane = threadIdx.x & 31;
+    int32_t top_e[4] = {0, 0, 0, 0}, top_n[4] = {0, 0, 0, 0};
+    for (int64_t c0 = static_cast<int64_t>(blockIdx.x) * kBinTile; c0 < n;
+         c0 += static_cast<int64_t>(gridDim.x) * kBinTile) {
+        if (threadIdx.x < 4)
+            tile_count[threadIdx.x] = 0;
+        __syncthreads();
+        int bucket[4], place[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int64_t col = c0 + u * kBinThreads + threadIdx.x;
+            int b = -1;
+            if (col < n && col >= rule.lo && col < rule.hi &&  // the requested column range
+                !(rule.rep && rule.rep[col] != col)) {         // solved by its representative
+                // sizes after at most ns pattern updates
+                const int64_t nf = static_cast<int64_t>(nk[col]) + rule.grow_n;
+                const int64_t ef = static_cast<int64_t>(E[col]) + rule.grow_e;
+                if (rule.small_list > 0 && ef <= kSmallE && nf <= kSmallN)
+                    b = 2;
+                else if (rule.single_bucket >= 0)
+                    b = rule.single_bucket;
+                else if (rule.allow_warp && ef <= rule.warp_emax && nf <= rule.warp_nmax)
+                    b = 0;
+                else if (rule.tiny_list > 0 && ef <= rule.tiny_emax && nf <= rule.tiny_nmax)
+                    b = 3;
+                else {
+                    const int64_t mw = ef / 2 + nf;
+                    const int64_t wbytes = (mw * nf + mw) * rule.elem_bytes;
+                    b = (wbytes <= rule.smem_w_bytes) ? 1 : 2;
+                }
+#pragma unroll
+                for (int x = 0; x < 4; x++) {
+                    if (b == x) {
+                        top_e[x] = max(top_e[x], static_cast<int32_t>(
+                                                     ef > 0x7fffffff ? 0x7fffffff : ef));
+                        top_n[x] = max(top_n[x], static_cast<int32_t>(nf));
+                    }
+                }
+            }
+            bucket[u] = b;
+            place[u] = 0;
+#pragma unroll
+            for (int x = 0; x < 4; x++) {
+                const uint32_t m = __ballot_sync(0xffffffffu, b == x);
+                if (m == 0)
+                    continue;
+                int base = 0;
+                if (lane == __ffs(m) - 1)
+                    base = atomicAdd(&tile_count[x], __popc(m));
+                base = __shfl_sync(0xffffffffu, base, __ffs(m) - 1);
+                if (b == x)
+                    place[u] = base + __popc(m & ((1u << lane) - 1u));
+            }
         }
-        const int slot = atomicAdd(&counts[b], 1);
-        lists[static_cast<int64_t>(b == 3 ? rule.tiny_list : b) * n + slot] = col;
-        atomicMax(&maxE[b], static_cast<int32_t>(ef > 0x7fffffff ? 0x7fffffff : ef));
-        atomicMax(&maxN[b], static_cast<int32_t>(nf));
+        __syncthreads();
+        if (threadIdx.x < 4 && tile_count[threadIdx.x] > 0)
+            tile_base[threadIdx.x] = atomicAdd(&counts[threadIdx.x], tile_count[threadIdx.x]);
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int b = bucket[u];
+            if (b < 0)
+                continue;
+            const int to =
+                b == 3 ? rule.tiny_list : (b == 2 && rule.small_list > 0 ? rule.small_list : b);
+            lists[static_cast<int64_t>(to) * n + tile_base[b] + place[u]] =
+                static_cast<int32_t>(c0 + u * kBinThreads + threadIdx.x);
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int x = 0; x < 4; x++) {
+        const int e = __reduce_max_sync(0xffffffffu, top_e[x]);
+        const int m = __reduce_max_sync(0xffffffffu, top_n[x]);
+        if (lane == 0 && (e > 0 || m > 0)) {
+            atomicMax(&maxE[x], e);
+            atomicMax(&maxN[x], m);
+        }
     }
 }
 
@@ -399,8 +467,8 @@ cudaError_t launch_plan(const int64_t* cptr, const int64_t* pptr, const int32_t*
     if (nprob <= 0)
         return cudaSuccess;
     const int threads = 256;
-    int blocks = (nprob + 7) / 8;
-    blocks = std::min(blocks, num_sms() * 16);
+    int blocks = (nprob + 31) / 32;
+    blocks = std::min(blocks, num_sms() * 8);
     plan_kernel<<<blocks, threads, 0, st>>>(cptr, pptr, pidx, nprob, bs, E, nk);
     return cudaGetLastError();
 }
@@ -411,8 +479,8 @@ cudaError_t launch_bucket(const int32_t* E, const int32_t* nk, int n, const Buck
 {
     if (n <= 0)
         return cudaSuccess;
-    int blocks = std::min((n + 255) / 256, num_sms() * 8);
-    bucket_kernel<<<blocks, 256, 0, st>>>(E, nk, n, rule, counts, maxE, maxN, lists);
+    int blocks = std::min((n + kBinTile - 1) / kBinTile, num_sms() * 4);
+    bucket_kernel<<<blocks, kBinThreads, 0, st>>>(E, nk, n, rule, counts, maxE, maxN, lists);
     return cudaGetLastError();
 }
 

@@ -25,6 +25,8 @@ struct BucketRule {
     int grow_e;            // mn * ns * max column nnz of C
     const int32_t* rep;    // reuse table: columns with rep[k] != k are skipped (nullable)
     int lo, hi;            // only problem columns [lo, hi) are binned
+    int small_list;        // > 0: work list of bucket 2, columns of at most eight unknowns
+                           // and 64 entries (small_qr.cu)
     int tiny_list;         // > 0: work list of bucket 3, small columns of the sparse
     int tiny_nmax;         // solver: |J| and
     int tiny_emax;         // entries of C(:,J) at most these
@@ -93,6 +95,13 @@ cudaError_t launch_fixed_solve(int elem_bytes, int arena_bytes, const Problem& p
                                int count_host, int32_t* counter, int32_t* ovf_list,
                                int32_t* ovf_count, void* rglob, int64_t rglob_elems, int max_ctas,
                                cudaStream_t st, int* grid_out);
+// Columns of at most eight unknowns and 64 entries of C(:, J) (small_qr.cu):
+// FP64 Householder QR, eight lanes per column.  rest (count entries) and
+// rest_count[2] (zero) are scratch.
+constexpr int kSmallN = 8;
+constexpr int kSmallE = 64;
+cudaError_t launch_small_qr(const Problem& pb, const Output& out, const int32_t* list, int count,
+                            int32_t* rest, int32_t* rest_count, cudaStream_t st);
 // Solvers on the sparse normal equations (fixed_cg.cu), a CTA per column in
 // slot_bytes of shared memory; the columns that one does not take go to
 // ovf_list / *ovf_count (appended).  nnz(C) < 2^32.
@@ -159,10 +168,16 @@ struct AdjointIO {
 // E[k], nk[k] of problem column k from the result's pattern
 cudaError_t launch_adjoint_plan(const int64_t* cptr, const int64_t* mptr, const int32_t* midx,
                                 int nprob, int bs, int32_t* E, int32_t* nk, cudaStream_t st);
-// problem columns [lo, hi) of the last setup
-cudaError_t launch_adjoint(const Problem& pb, const Caps& cap, const AdjointIO& io, int lo,
-                           int hi, bool warp, char* scratch, size_t scratch_bytes,
-                           int32_t* counter, cudaStream_t st);
+// problem columns list[0 .. count)
+cudaError_t launch_adjoint(const Problem& pb, const Caps& cap, const AdjointIO& io,
+                           const int32_t* list, int count, bool warp, char* scratch,
+                           size_t scratch_bytes, int32_t* counter, cudaStream_t st);
 size_t adjoint_scratch_bytes(const Caps& cap, int n, bool warp);
+// scalar columns of at most eight unknowns without a gbar: eight lanes each
+cudaError_t launch_adjoint_small(const Problem& pb, const AdjointIO& io, const int32_t* list,
+                                 int count, cudaStream_t st);
+// *total = sum of v[0 .. n), compensated, in a fixed order; tmp: kLossParts pairs
+constexpr int kLossParts = 1024;
+cudaError_t launch_loss_sum(const double* v, int n, double* tmp, double* total, cudaStream_t st);
 
 }  // namespace mspai
