@@ -44,9 +44,11 @@ __device__ void adj_apply_c(const G& g, const Slot<double>& s, int m, const doub
 
 // lambda (in gv) = (C^T C)^-1 gbar with the kept R (packed by columns, TR):
 // two triangular solves, then FP64 refinement steps gv += R^-1 R^-T (gbar -
-// C^T C gv) when TR is FP32.  q (m entries) and tmp (n) are scratch.
+// C^T C gv) until the correction is below 2^-44 of lambda (R may be FP32, or
+// of values before a re-setup).  q (m entries) and tmp (n) are scratch.
+// Returns (group-uniformly) false when the corrections do not get there.
 template <class TR, class G>
-__device__ void adj_lambda_kept(const G& g, const Slot<double>& s, const TR* R, int m, int n,
+__device__ bool adj_lambda_kept(const G& g, const Slot<double>& s, const TR* R, int m, int n,
                                 const double* gbar, double* gv, double* q, double* tmp)
 {
     for (int jj = g.rank(); jj < n; jj += G::kSize)
@@ -54,8 +56,8 @@ __device__ void adj_lambda_kept(const G& g, const Slot<double>& s, const TR* R, 
     g.sync();
     const RView<TR> rv{R, 0};
     group_normal_correction_blocked<TR>(g, rv, n, gv);
-    const int steps = sizeof(TR) == 4 ? 2 : 0;
-    for (int it = 0; it < steps; it++) {
+    double d2_prev = 0.0;
+    for (int it = 0; it < 24; it++) {
         adj_apply_c(g, s, m, gv, q);
         // tmp = gbar - C^T q, a warp per column over its entries
         for (int jj = g.warp(); jj < n; jj += G::kWarps) {
@@ -68,10 +70,23 @@ __device__ void adj_lambda_kept(const G& g, const Slot<double>& s, const TR* R, 
         }
         g.sync();
         group_normal_correction_blocked<TR>(g, rv, n, tmp);
-        for (int jj = g.rank(); jj < n; jj += G::kSize)
-            gv[jj] += tmp[jj];
+        double d2 = 0.0, x2 = 0.0;
+        for (int jj = g.rank(); jj < n; jj += G::kSize) {
+            const double v = gv[jj] + tmp[jj];
+            gv[jj] = v;
+            d2 += tmp[jj] * tmp[jj];
+            x2 += v * v;
+        }
+        d2 = g.sum(d2);
+        x2 = g.sum(x2);
         g.sync();
+        if (d2 <= 0x1p-88 * x2)
+            return true;
+        if (it > 0 && !(d2 <= 0.25 * d2_prev))
+            return false;
+        d2_prev = d2;
     }
+    return false;
 }
 
 template <class TR, class G>
@@ -147,11 +162,8 @@ __device__ void adjoint_column(const G& g, const Problem& pb, const Caps& cap, S
         const double* gb = io.gbar + io.mptr[kb];
         for (int jj = g.rank(); jj < n; jj += G::kSize)
             gx += gb[jj] * s.x[jj];
-        if (io.rstore) {
-            adj_lambda_kept<TR>(g, s, static_cast<const TR*>(io.rstore) + io.roff[kb], m, n, gb,
-                                s.gv, q, s.rinv);
-        }
-        else {
+        if (!io.rstore || !adj_lambda_kept<TR>(g, s, static_cast<const TR*>(io.rstore) + io.roff[kb],
+                                               m, n, gb, s.gv, q, s.rinv)) {
             // recompute R: the folded Householder QR of the forward, in FP64
             for (int u = g.rank(); u < m; u += G::kSize)
                 s.tmp[u] = (s.rstart[u + 1] - s.rstart[u]) >= 2 ? 1 : 0;

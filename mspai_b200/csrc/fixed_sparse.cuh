@@ -123,7 +123,10 @@ struct SharedEntries {
     double* gd;           // squares of all entries
     double* us;           // n values
     double* xs;           // n values: the solution, by position
-    uint16_t* ccol;       // column of J at each position (decreasing shared entries)
+    uint32_t* cb;         // start of C(:, J(i))
+    uint32_t* tmp;        // n words
+    uint16_t* cpos;       // position of each column of J (decreasing shared entries)
+    uint16_t* ccol;       // column of J at each position
     double* ev;           // shared entries by row: value and position of the column
     uint16_t* ec;
     double* cv;           // by column: value and row number
@@ -578,6 +581,9 @@ __device__ bool gather_shared(CgShared& sh, const Problem& pb, int col, char* ba
     g.gd = gd;
     g.us = us;
     g.xs = xs;
+    g.cb = cb;
+    g.tmp = clen;
+    g.cpos = cpos;
     g.ccol = ccol;
     g.ev = ev;
     g.ec = ec;

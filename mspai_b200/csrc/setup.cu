@@ -682,10 +682,13 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
     const bool small = use_fixed && !out.rstore;
     rule.small_list = small ? kLists + 3 : 0;
     // small fixed columns: a list of their own for the sparse solvers
-    const bool sparse = use_fixed && !out.rstore && C->nnz < (int64_t(1) << 32) &&
+    // (a re-setup starts them from M's values; where the factors are to be made
+    // they have none to keep)
+    const bool sparse = use_fixed && (!out.rstore || reuse_now) &&
+                        C->nnz < (int64_t(1) << 32) &&
                         (elem == 8 || pb.refine > 0) &&
                         kSparseClasses[0].slot_bytes <= h->fixed_arena;
-    rule.tiny_list = sparse ? kLists + 2 : 0;
+    rule.tiny_list = sparse && !out.rstore ? kLists + 2 : 0;
     rule.tiny_nmax = kSparseTinyN;
     rule.tiny_emax = kSparseTinyE;
     rule.elem_bytes = elem;
@@ -744,7 +747,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
         h->stats.bucket_columns[0] = nsmall;
     }
     h->small_len = nsmall;
-    const int tiny = sparse ? hc[3] : 0;  // small columns of the sparse solvers
+    const int tiny = rule.tiny_list > 0 ? hc[3] : 0;  // small columns of the sparse solvers
     h->tiny_len = tiny;
     if (tiny > 0) {  // their sizes belong to the fixed-pattern bucket
         hc[4 + 1] = std::max(hc[4 + 1], hc[4 + 3]);
@@ -827,9 +830,8 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
                                           mspai::fixed_max_grid(h->fixed_arena_large));
             CUDA_TRY(h, h->rglob.ensure(static_cast<size_t>(grid_max) * relems * elem));
             CUDA_TRY(h, cudaEventRecord(h->evb[2], st));
-            // the sparse normal equations first (no factor to keep; the slots
-            // count against the first launch's arena), the rest to the dense
-            // factorizations
+            // the sparse normal equations first (their slots count against the
+            // first launch's arena), the rest to the dense factorizations
             const int32_t* flist = list;
             const int32_t* fcount = nullptr;
             if (sparse) {
@@ -1336,7 +1338,27 @@ extern "C" int mspai_adjoint_weighted(mspai_handle* h, const mspai_csc* C, const
                         pb, io, h->lists.as<int32_t>() + 2 * static_cast<size_t>(nprob), hc[2],
                         st));
     }
-    if (hc[0] > 0) {
+    // larger scalar columns: the sparse form of their problem; what it leaves
+    // (counted on the host) goes to the general adjoint
+    const int32_t* alist = h->lists.as<int32_t>();
+    int acount = hc[0];
+    if (acount > 0 && bs == 1 && C->nnz < (int64_t(1) << 32) && hc[4] > 64) {
+        Problem pm = pb;
+        pm.pptr = io.mptr;
+        pm.pidx = io.midx;
+        int32_t* lists = h->lists.as<int32_t>();
+        int32_t* const rest[2] = {lists + static_cast<size_t>(nprob),
+                                  lists + 2 * static_cast<size_t>(nprob)};
+        int32_t *left = nullptr, *left_count = nullptr;
+        h->launches += 3;
+        CUDA_TRY(h, mspai::launch_adjoint_sparse(pm, io, alist, acount, rest, dcnt + 32, &left,
+                                                 &left_count, st));
+        CUDA_TRY(h, cudaMemcpyAsync(&acount, left_count, sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                    st));
+        CUDA_TRY(h, cudaStreamSynchronize(st));
+        alist = left;
+    }
+    if (acount > 0) {
         Caps cap{};
         cap.emax = std::max(1, hc[4]);
         cap.nmax = std::max(1, hc[8]);
@@ -1347,11 +1369,11 @@ extern "C" int mspai_adjoint_weighted(mspai_handle* h, const mspai_csc* C, const
         cap.nrhs = bs;
         cap.nbmap = 0;
         const bool warp = cap.emax <= 64 && cap.nmax <= 16;
-        const size_t need = mspai::adjoint_scratch_bytes(cap, hc[0], warp);
+        const size_t need = mspai::adjoint_scratch_bytes(cap, acount, warp);
         CUDA_TRY(h, h->scratch.ensure(need));
         CUDA_TRY(h, cudaMemsetAsync(dcnt + 20, 0, sizeof(int32_t), st));
         h->launches++;
-        CUDA_TRY(h, mspai::launch_adjoint(pb, cap, io, h->lists.as<int32_t>(), hc[0], warp,
+        CUDA_TRY(h, mspai::launch_adjoint(pb, cap, io, alist, acount, warp,
                                           h->scratch.as<char>(), h->scratch.bytes, dcnt + 20,
                                           st));
     }

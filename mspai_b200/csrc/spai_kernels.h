@@ -176,6 +176,12 @@ size_t adjoint_scratch_bytes(const Caps& cap, int n, bool warp);
 // scalar columns of at most eight unknowns without a gbar: eight lanes each
 cudaError_t launch_adjoint_small(const Problem& pb, const AdjointIO& io, const int32_t* list,
                                  int count, cudaStream_t st);
+// scalar columns on the sparse form of their problem (adjoint_sparse.cu; pb with
+// the result's pattern as P); what it leaves is *left[0 .. **left_count).  rest:
+// two lists of count entries; counts[6] (zero).  nnz(C) < 2^32.
+cudaError_t launch_adjoint_sparse(const Problem& pb, const AdjointIO& io, const int32_t* list,
+                                  int count, int32_t* const rest[2], int32_t* counts,
+                                  int32_t** left, int32_t** left_count, cudaStream_t st);
 // *total = sum of v[0 .. n), compensated, in a fixed order; tmp: kLossParts pairs
 constexpr int kLossParts = 1024;
 cudaError_t launch_loss_sum(const double* v, int n, double* tmp, double* total, cudaStream_t st);
