@@ -455,6 +455,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
         check_launches = k;
     }
     int max_row_nnz = 0, max_col_nnz = 0;
+    bool need_rows = false;  // the row structure of C is to be built
     if (adaptive) {
         std::vector<int64_t> rp;
         std::vector<int32_t> rc2;
@@ -476,40 +477,50 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             CUDA_TRY(h, fetch(rp, C_rows->colptr, C_rows->ncols + 1, C_rows->mem, st));
         }
         else {
-            // the row structure of C on the device: a stable radix sort of the
-            // entries by row keeps each row's columns ascending; rows below n
-            // are a prefix of it (the probing rows come last)
-            const int nr = C->nrows;
-            const int64_t nz = C->nnz;
-            const size_t tb = mspai::rows_build_temp_bytes(nz, nr);
-            CUDA_TRY(h, h->rptr.ensure(sizeof(int64_t) * (static_cast<size_t>(nr) + 1)));
-            CUDA_TRY(h, h->rcol.ensure(sizeof(int32_t) * std::max<int64_t>(nz, 1)));
-            CUDA_TRY(h, h->tkeys.ensure(sizeof(int32_t) * std::max<int64_t>(nz, 1)));
-            CUDA_TRY(h, h->tperm0.ensure(sizeof(int32_t) * std::max<int64_t>(nz, 1)));
-            CUDA_TRY(h, h->tperm1.ensure(sizeof(int32_t) * std::max<int64_t>(nz, 1)));
-            CUDA_TRY(h, h->tcnt.ensure(sizeof(int32_t) * std::max(nr, 1)));
-            CUDA_TRY(h, h->ttemp.ensure(std::max<size_t>(tb, 16)));
-            CUDA_TRY(h, h->scan_tmp.ensure(sizeof(int64_t) * ((nr + 1023) / 1024 + 2)));
-            h->launches += 7;
-            CUDA_TRY(h, mspai::launch_build_rows(
-                            pb.cptr, pb.cidx, nullptr, n, nr, nz, h->rptr.as<int64_t>(),
-                            h->rcol.as<int32_t>(), nullptr, h->tkeys.as<int32_t>(),
-                            h->tperm0.as<int32_t>(), h->tperm1.as<int32_t>(),
-                            h->tcnt.as<int32_t>(), h->scan_tmp.as<int64_t>(), h->ttemp.p,
-                            h->ttemp.bytes, st));
-            pb.rptr = h->rptr.as<int64_t>();
-            pb.rcol = h->rcol.as<int32_t>();
-            CUDA_TRY(h, h->counters.ensure(64 * sizeof(int32_t)));
-            int32_t* mx = h->counters.as<int32_t>() + 17;
-            h->launches++;
-            CUDA_TRY(h, mspai::launch_max_len(pb.rptr, n, mx, st));
-            CUDA_TRY(h, cudaMemcpyAsync(&max_row_nnz, mx, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                        st));
-            CUDA_TRY(h, cudaStreamSynchronize(st));
+            need_rows = true;
         }
         for (size_t i = 0; i + 1 < rp.size(); i++)
             max_row_nnz = std::max<int>(max_row_nnz, static_cast<int>(rp[i + 1] - rp[i]));
     }
+    // builds it (blocks: only when a column needs a pattern update)
+    auto build_rows = [&]() -> int {
+        // the row structure of C on the device: a stable radix sort of the
+        // entries by row keeps each row's columns ascending; rows below n
+        // are a prefix of it (the probing rows come last)
+        const int nr = C->nrows;
+        const int64_t nz = C->nnz;
+        const size_t tb = mspai::rows_build_temp_bytes(nz, nr);
+        CUDA_TRY(h, h->rptr.ensure(sizeof(int64_t) * (static_cast<size_t>(nr) + 1)));
+        CUDA_TRY(h, h->rcol.ensure(sizeof(int32_t) * std::max<int64_t>(nz, 1)));
+        CUDA_TRY(h, h->tkeys.ensure(sizeof(int32_t) * std::max<int64_t>(nz, 1)));
+        CUDA_TRY(h, h->tperm0.ensure(sizeof(int32_t) * std::max<int64_t>(nz, 1)));
+        CUDA_TRY(h, h->tperm1.ensure(sizeof(int32_t) * std::max<int64_t>(nz, 1)));
+        CUDA_TRY(h, h->tcnt.ensure(sizeof(int32_t) * std::max(nr, 1)));
+        CUDA_TRY(h, h->ttemp.ensure(std::max<size_t>(tb, 16)));
+        CUDA_TRY(h, h->scan_tmp.ensure(sizeof(int64_t) * ((nr + 1023) / 1024 + 2)));
+        h->launches += 7;
+        CUDA_TRY(h, mspai::launch_build_rows(
+                        pb.cptr, pb.cidx, nullptr, n, nr, nz, h->rptr.as<int64_t>(),
+                        h->rcol.as<int32_t>(), nullptr, h->tkeys.as<int32_t>(),
+                        h->tperm0.as<int32_t>(), h->tperm1.as<int32_t>(),
+                        h->tcnt.as<int32_t>(), h->scan_tmp.as<int64_t>(), h->ttemp.p,
+                        h->ttemp.bytes, st));
+        pb.rptr = h->rptr.as<int64_t>();
+        pb.rcol = h->rcol.as<int32_t>();
+        CUDA_TRY(h, h->counters.ensure(64 * sizeof(int32_t)));
+        int32_t* mx = h->counters.as<int32_t>() + 17;
+        h->launches++;
+        CUDA_TRY(h, mspai::launch_max_len(pb.rptr, n, mx, st));
+        CUDA_TRY(h, cudaMemcpyAsync(&max_row_nnz, mx, sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                    st));
+        CUDA_TRY(h, cudaStreamSynchronize(st));
+        return MSPAI_OK;
+    };
+    // block columns are first solved at their start pattern
+    const bool blocks = bs > 1 && prm->batched && C->nnz < (int64_t(1) << 32) &&
+                        (prm->prec != MSPAI_PREC_MIXED || prm->refine > 0);
+    if (need_rows && !blocks && (rc = build_rows()) != MSPAI_OK)
+        return rc;
     pb.bs = bs;
     pb.ep = prm->ep;
     pb.mn = prm->mn;
@@ -676,7 +687,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
     // fixed scalar patterns: every column beyond the warp bucket goes to the
     // fixed-pattern solver (bucket 1), which sizes its arrays per column
     const bool use_fixed = !adaptive && bs == 1 && prm->batched && !pb.qru;
-    rule.smem_w_bytes = use_fixed ? (int64_t(1) << 62) : h->w_smem_bytes;
+    rule.smem_w_bytes = (use_fixed || blocks) ? (int64_t(1) << 62) : h->w_smem_bytes;
     // the smallest fixed columns: eight lanes each (the store of R holds one
     // element type, the small QR is FP64: not when R is kept)
     const bool small = use_fixed && !out.rstore;
@@ -780,6 +791,34 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
         int32_t* list = h->lists.as<int32_t>() + static_cast<size_t>(b) * nprob;
         int32_t* counter = dcnt + 12 + b;
         CUDA_TRY(h, cudaMemsetAsync(counter, 0, sizeof(int32_t), st));
+        int left = count;  // columns for the solver below
+        if (blocks) {
+            int32_t* lists = h->lists.as<int32_t>();
+            int32_t* rest = lists + static_cast<size_t>(kLists + 1) * nprob;
+            int32_t* bc = dcnt + 28;
+            CUDA_TRY(h, cudaMemsetAsync(bc, 0, 4 * sizeof(int32_t), st));
+            CUDA_TRY(h, cudaEventRecord(h->evb[2 * b], st));
+            h->launches += 2;
+            CUDA_TRY(h, mspai::launch_block_solve(elem, pb, out, list, count,
+                                                  lists + static_cast<size_t>(kLists) * nprob,
+                                                  rest, bc, st));
+            CUDA_TRY(h, cudaEventRecord(h->evb[2 * b + 1], st));
+            timed[b] = true;
+            h->stats.bucket_columns[b] = count;
+            CUDA_TRY(h, cudaMemcpyAsync(&left, bc + 1, sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                        st));
+            CUDA_TRY(h, cudaStreamSynchronize(st));
+            if (left == 0)
+                continue;
+            list = rest;
+            if (need_rows) {
+                if ((rc = build_rows()) != MSPAI_OK)
+                    return rc;
+                cap.cmax = static_cast<int>(std::min<int64_t>(
+                    nprob, static_cast<int64_t>(cap.emax + 1) * bs * std::max(1, max_row_nnz)));
+                cap.lcand = mspai::next_pow2(cap.cmax);
+            }
+        }
         int grid = 0;
         // small problems in mixed mode: FP64 without refinement (not when R
         // is kept: its store has one element type)
@@ -894,8 +933,9 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             }
         }
         else {
-            CUDA_TRY(h, cudaEventRecord(h->evb[2 * b], st));
-            const int rc2 = run_cta(b, cap, list, count, counter, h->smem_budget, elem_b, pbb);
+            if (!blocks)
+                CUDA_TRY(h, cudaEventRecord(h->evb[2 * b], st));
+            const int rc2 = run_cta(b, cap, list, left, counter, h->smem_budget, elem_b, pbb);
             if (rc2 != MSPAI_OK)
                 return rc2;
             CUDA_TRY(h, cudaEventRecord(h->evb[2 * b + 1], st));
