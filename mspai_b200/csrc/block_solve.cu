@@ -339,6 +339,230 @@ __device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Prob
     return true;
 }
 
+// Block columns of at most eight unknowns, FP64: eight lanes per column, four
+// columns per warp.  Lane j walks the sorted entries of C(:, J)'s column j and
+// lane c those of the target's column c; the smallest head is the next row.  The
+// first walk sums G = C^T C (lane j: its row) and C^T b, each further one forms
+// the residual row by row and C^T (b - C x) for the refinement, so that nothing
+// is stored.
+__device__ __forceinline__ double sum8(double v)
+{
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v;
+}
+
+__global__ void __launch_bounds__(128)
+    block_small_kernel(Problem pb, Output out, const int32_t* __restrict__ list, int count,
+                       int32_t* __restrict__ ovf_list, int32_t* __restrict__ ovf_count)
+{
+    constexpr uint32_t all = 0xffffffffu;
+    const int lane = threadIdx.x & 31, grp = lane >> 3, l8 = lane & 7;
+    const int bs = pb.bs;
+    const int warps = (gridDim.x * blockDim.x) >> 5;
+    const int most = pb.refine > 0 ? pb.refine + 2 : 3;
+    for (int64_t t0 = 4 * static_cast<int64_t>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+         t0 < count; t0 += 4 * static_cast<int64_t>(warps)) {
+        const int kb = t0 + grp < count ? list[t0 + grp] : -1;
+        int n = 0, col = 0;
+        int64_t a0 = 0, a1 = 0, q0 = 0, q1 = 0;
+        if (kb >= 0) {
+            const int64_t p0 = pb.pptr[kb];
+            n = bs * static_cast<int>(pb.pptr[kb + 1] - p0);
+            if (n > 8 || n < 1) {
+                n = 0;
+            }
+            else if (l8 < n) {
+                col = bs * pb.pidx[p0 + l8 / bs] + l8 % bs;
+                a0 = pb.cptr[col];
+                a1 = pb.cptr[col + 1];
+            }
+            if (pb.bptr && l8 < bs) {
+                q0 = pb.bptr[bs * kb + l8];
+                q1 = pb.bptr[bs * kb + l8 + 1];
+            }
+        }
+        bool live = n > 0;  // still a candidate
+        bool done = !live;  // converged, or left to the other kernels
+        const int nmax = __reduce_max_sync(all, n);
+        double G[8], lk[8], lt[8], linv = 0.0;
+        double x[8], gr[8];  // per right-hand side: this lane's unknown
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            G[i] = lk[i] = lt[i] = x[i] = gr[i] = 0.0;
+        double r2 = 0.0, d2_prev = 0.0;
+        int m = 0, solves = 0;
+        for (int it = 0;; it++) {
+            // ---- one walk over the rows
+            int64_t e = a0, q = q0;
+            int row = e < a1 ? __ldg(pb.cidx + e) : 0x7fffffff;
+            double val = e < a1 ? __ldg(pb.cval + e) : 0.0;
+            int brow = pb.bptr ? (q < q1 ? __ldg(pb.bidx + q) : 0x7fffffff)
+                               : (kb >= 0 && l8 < bs ? bs * kb + l8 : 0x7fffffff);
+            double part = 0.0;
+#pragma unroll
+            for (int c = 0; c < 8; c++)
+                gr[c] = 0.0;
+            while (true) {
+                int low = min(row, __shfl_xor_sync(all, row, 4));
+                low = min(low, __shfl_xor_sync(all, low, 2));
+                low = min(low, __shfl_xor_sync(all, low, 1));
+                const bool more = low != 0x7fffffff;
+                if (!__any_sync(all, more))
+                    break;
+                const bool mine = more && row == low;
+                const double v = mine ? val : 0.0;
+                if (pb.bptr)
+                    while (more && brow < low) {
+                        q++;
+                        brow = q < q1 ? __ldg(pb.bidx + q) : 0x7fffffff;
+                    }
+                const double b = (more && brow == low) ? (pb.bptr ? __ldg(pb.bval + q) : 1.0) : 0.0;
+                if (it == 0) {
+                    m += more ? 1 : 0;
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+                        if (i < nmax)
+                            G[i] += v * __shfl_sync(all, v, i, 8);
+                }
+#pragma unroll
+                for (int c = 0; c < 8; c++) {
+                    if (c < bs) {
+                        double r = __shfl_sync(all, b, c, 8);
+                        if (it > 0)
+                            r -= sum8(v * x[c]);
+                        gr[c] += v * r;
+                        part += r * r;
+                    }
+                }
+                if (mine) {
+                    e++;
+                    row = e < a1 ? __ldg(pb.cidx + e) : 0x7fffffff;
+                    val = e < a1 ? __ldg(pb.cval + e) : 0.0;
+                }
+            }
+            r2 = part;
+            if (it == 0) {
+                // ---- Cholesky, a lane per row: lk its row of L, lt its column
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    if (k >= nmax)
+                        break;
+                    const double piv = __shfl_sync(all, G[k], k, 8);
+                    const bool in = k < n;
+                    if (in && !(piv > 0.0))
+                        done = true, live = false;
+                    const double inv = in && piv > 0.0 ? 1.0 / sqrt(piv) : 0.0;
+                    if (l8 == k)
+                        linv = inv;
+                    const double l = l8 > k ? G[k] * inv : 0.0;
+                    lk[k] = l;
+#pragma unroll
+                    for (int i = 0; i < 8; i++) {
+                        if (i > k && i < nmax) {
+                            const double li = __shfl_sync(all, l, i, 8);
+                            G[i] -= l * li;
+                            if (l8 == k)
+                                lt[i] = li;
+                        }
+                    }
+                }
+            }
+            // this walk only gave the residual of the converged columns
+            if (__all_sync(all, done))
+                break;
+            // ---- x += G^-1 gr
+            double d2 = 0.0, x2 = 0.0;
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                if (c >= bs)
+                    break;
+                double z = gr[c];
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    if (k >= nmax)
+                        break;
+                    if (l8 == k)
+                        z *= linv;
+                    const double zk = __shfl_sync(all, z, k, 8);
+                    if (l8 > k)
+                        z -= lk[k] * zk;
+                }
+#pragma unroll
+                for (int k = 7; k >= 0; k--) {
+                    if (k >= nmax)
+                        continue;
+                    if (l8 == k)
+                        z *= linv;
+                    const double zk = __shfl_sync(all, z, k, 8);
+                    if (l8 < k)
+                        z -= lt[k] * zk;
+                }
+                if (!done && l8 < n) {
+                    x[c] += z;
+                    d2 += z * z;
+                    x2 += x[c] * x[c];
+                }
+            }
+            d2 = sum8(d2);
+            x2 = sum8(x2);
+            if (!done) {
+                solves++;
+                if (d2 <= 0x1p-88 * x2) {
+                    done = true;
+                }
+                else if (it + 1 == most || (it > 0 && !(d2 <= 0.25 * d2_prev)) ||
+                         (it == 1 && pb.refine == 0)) {
+                    done = true;
+                    live = false;
+                }
+                d2_prev = d2;
+            }
+        }
+        const double res = sqrt(r2);
+        if (pb.ns > 0 && !(res <= pb.ep * sqrt(static_cast<double>(bs))))
+            live = false;
+        int entries = static_cast<int>(a1 - a0);
+        entries += __shfl_xor_sync(all, entries, 4);
+        entries += __shfl_xor_sync(all, entries, 2);
+        entries += __shfl_xor_sync(all, entries, 1);
+        if (kb >= 0 && !live && l8 == 0)
+            ovf_list[atomicAdd(ovf_count, 1)] = kb;
+#pragma unroll
+        for (int c = 0; c < 8; c++) {
+            if (c >= bs)
+                break;
+            const uint32_t odd = __ballot_sync(all, l8 < n && !isfinite(x[c]));
+            if (!live)
+                continue;
+            const int sc = bs * kb + c;
+            const int64_t o0 = out.optr[sc];
+            if (l8 < n) {
+                out.oval[o0 + l8] = x[c];
+                if (out.write_idx)
+                    out.oidx[o0 + l8] = col;
+            }
+            if (l8 == 0) {
+                const bool bad = ((odd >> (8 * grp)) & 0xffu) != 0 || !isfinite(res);
+                out.olen[sc] = n;
+                out.res[sc] = res;
+                out.steps[sc] = 1;
+                out.status[sc] = bad ? 2 : 0;
+            }
+        }
+        if (live && l8 == 0) {
+            const double dn = n, dm = m, dr = bs, E = entries;
+            double* wk = out.work + 3 * static_cast<size_t>(kb);
+            wk[0] += dn * E + dn * dn * dn / 3.0 + solves * dr * (2.0 * dn * dn + 4.0 * E);
+            wk[1] += 2.0 * dm * dn * dn - (2.0 / 3.0) * dn * dn * dn + 4.0 * dm * dn * dr +
+                     2.0 * dm * dn * dr;
+            wk[2] += 12.0 * E + 16.0 * dn + 8.0 * dm * dr;
+        }
+        __syncwarp();
+    }
+}
+
 template <class T, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     block_solve_kernel(Problem pb, Output out, const int32_t* __restrict__ list,
@@ -390,20 +614,25 @@ cudaError_t launch_block_t(int arena, const Problem& pb, const Output& out, cons
 }  // namespace
 
 cudaError_t launch_block_solve(int elem_bytes, const Problem& pb, const Output& out,
-                               const int32_t* list, int count, int32_t* between, int32_t* rest,
+                               const int32_t* list, int count, int32_t* const rest[2],
                                int32_t* counts, cudaStream_t st)
 {
-    // small columns in FP64 (no refinement to speak of on a few unknowns), 64
-    // threads; then 256 threads and two CTAs per SM, in FP64 one
-    cudaError_t e = launch_block_t<double, 64, 12>(15 * 1024, pb, out, list, nullptr, count,
-                                                   counts + 2, between, counts, st);
+    // at most eight unknowns: eight lanes; small columns in FP64 (no refinement
+    // to speak of on a few unknowns), 64 threads; then 256 threads and two CTAs
+    // per SM, in FP64 one
+    const int blocks = std::max(1, std::min((count + 15) / 16, num_sms() * 16));
+    block_small_kernel<<<blocks, 128, 0, st>>>(pb, out, list, count, rest[0], counts);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+        e = launch_block_t<double, 64, 12>(15 * 1024, pb, out, rest[0], counts, count, counts + 3,
+                                           rest[1], counts + 1, st);
     if (e != cudaSuccess)
         return e;
     if (elem_bytes == 4)
-        return launch_block_t<float, 256, 2>(107 * 1024, pb, out, between, counts, count,
-                                             counts + 3, rest, counts + 1, st);
-    return launch_block_t<double, 256, 1>(212 * 1024, pb, out, between, counts, count, counts + 3,
-                                          rest, counts + 1, st);
+        return launch_block_t<float, 256, 2>(107 * 1024, pb, out, rest[1], counts + 1, count,
+                                             counts + 4, rest[0], counts + 2, st);
+    return launch_block_t<double, 256, 1>(212 * 1024, pb, out, rest[1], counts + 1, count,
+                                          counts + 4, rest[0], counts + 2, st);
 }
 
 }  // namespace mspai

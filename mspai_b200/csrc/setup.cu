@@ -794,23 +794,22 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
         int left = count;  // columns for the solver below
         if (blocks) {
             int32_t* lists = h->lists.as<int32_t>();
-            int32_t* rest = lists + static_cast<size_t>(kLists + 1) * nprob;
+            int32_t* const rest[2] = {lists + static_cast<size_t>(kLists) * nprob,
+                                      lists + static_cast<size_t>(kLists + 1) * nprob};
             int32_t* bc = dcnt + 28;
-            CUDA_TRY(h, cudaMemsetAsync(bc, 0, 4 * sizeof(int32_t), st));
+            CUDA_TRY(h, cudaMemsetAsync(bc, 0, 5 * sizeof(int32_t), st));
             CUDA_TRY(h, cudaEventRecord(h->evb[2 * b], st));
-            h->launches += 2;
-            CUDA_TRY(h, mspai::launch_block_solve(elem, pb, out, list, count,
-                                                  lists + static_cast<size_t>(kLists) * nprob,
-                                                  rest, bc, st));
+            h->launches += 3;
+            CUDA_TRY(h, mspai::launch_block_solve(elem, pb, out, list, count, rest, bc, st));
             CUDA_TRY(h, cudaEventRecord(h->evb[2 * b + 1], st));
             timed[b] = true;
             h->stats.bucket_columns[b] = count;
-            CUDA_TRY(h, cudaMemcpyAsync(&left, bc + 1, sizeof(int32_t), cudaMemcpyDeviceToHost,
+            CUDA_TRY(h, cudaMemcpyAsync(&left, bc + 2, sizeof(int32_t), cudaMemcpyDeviceToHost,
                                         st));
             CUDA_TRY(h, cudaStreamSynchronize(st));
             if (left == 0)
                 continue;
-            list = rest;
+            list = rest[0];
             if (need_rows) {
                 if ((rc = build_rows()) != MSPAI_OK)
                     return rc;

@@ -115,12 +115,12 @@ cudaError_t launch_sparse_solve(int elem_bytes, SparseLaunch kind, int slot_byte
                                 const Problem& pb, const Output& out, const int32_t* list,
                                 const int32_t* count_dev, int count_host, int32_t* counter,
                                 int32_t* ovf_list, int32_t* ovf_count, cudaStream_t st);
-// Block columns at their start pattern (block_solve.cu); rest / counts[1]: the
+// Block columns at their start pattern (block_solve.cu); rest[0] / counts[2]: the
 // columns left to the general solver (with pattern updates also those whose
-// residual is above the tolerance).  between: a list of count entries;
-// counts[4] (zero).  nnz(C) < 2^32.
+// residual is above the tolerance).  rest: two lists of count entries;
+// counts[5] (zero).  nnz(C) < 2^32.
 cudaError_t launch_block_solve(int elem_bytes, const Problem& pb, const Output& out,
-                               const int32_t* list, int count, int32_t* between, int32_t* rest,
+                               const int32_t* list, int count, int32_t* const rest[2],
                                int32_t* counts, cudaStream_t st);
 cudaError_t launch_scan_lengths(const int32_t* len, int n, int64_t* ptr, int64_t* tmp,
                                 cudaStream_t st);
