@@ -398,6 +398,9 @@ __global__ void __launch_bounds__(128)
             int64_t e = a0, q = q0;
             int row = e < a1 ? __ldg(pb.cidx + e) : 0x7fffffff;
             double val = e < a1 ? __ldg(pb.cval + e) : 0.0;
+            // the entry after it, on its way while a row is worked on
+            int next_row = e + 1 < a1 ? __ldg(pb.cidx + e + 1) : 0x7fffffff;
+            double next_val = e + 1 < a1 ? __ldg(pb.cval + e + 1) : 0.0;
             int brow = pb.bptr ? (q < q1 ? __ldg(pb.bidx + q) : 0x7fffffff)
                                : (kb >= 0 && l8 < bs ? bs * kb + l8 : 0x7fffffff);
             double part = 0.0;
@@ -438,8 +441,10 @@ __global__ void __launch_bounds__(128)
                 }
                 if (mine) {
                     e++;
-                    row = e < a1 ? __ldg(pb.cidx + e) : 0x7fffffff;
-                    val = e < a1 ? __ldg(pb.cval + e) : 0.0;
+                    row = next_row;
+                    val = next_val;
+                    next_row = e + 1 < a1 ? __ldg(pb.cidx + e + 1) : 0x7fffffff;
+                    next_val = e + 1 < a1 ? __ldg(pb.cval + e + 1) : 0.0;
                 }
             }
             r2 = part;

@@ -71,6 +71,9 @@ __global__ void __launch_bounds__(kSmallThreads)
         entries += __shfl_xor_sync(kAll, entries, 1);
         int row = e < e1 ? __ldg(pb.cidx + e) : 0x7fffffff;
         double val = e < e1 ? __ldg(pb.cval + e) : 0.0;
+        // the entry after it, on its way while a row is worked on
+        int next_row = e + 1 < e1 ? __ldg(pb.cidx + e + 1) : 0x7fffffff;
+        double next_val = e + 1 < e1 ? __ldg(pb.cval + e + 1) : 0.0;
         int m = 0;
         while (true) {
             int low = min(row, __shfl_xor_sync(kAll, row, 4));
@@ -88,8 +91,10 @@ __global__ void __launch_bounds__(kSmallThreads)
             m += more ? 1 : 0;
             if (mine) {
                 e++;
-                row = e < e1 ? __ldg(pb.cidx + e) : 0x7fffffff;
-                val = e < e1 ? __ldg(pb.cval + e) : 0.0;
+                row = next_row;
+                val = next_val;
+                next_row = e + 1 < e1 ? __ldg(pb.cidx + e + 1) : 0x7fffffff;
+                next_val = e + 1 < e1 ? __ldg(pb.cval + e + 1) : 0.0;
             }
         }
         const bool fits = m <= M;

@@ -289,17 +289,51 @@ __global__ void scan_add_kernel(int64_t* __restrict__ out, int n, const int64_t*
         out[i] += block_off[blockIdx.x];
 }
 
-__global__ void scan_serial_kernel(int64_t* __restrict__ v, int nb)
+// Exclusive scan of the block sums by one CTA, 1024 at a time (one thread took
+// 25 us for the 192 sums of 192,000 columns).
+__global__ void __launch_bounds__(1024) scan_sums_kernel(int64_t* __restrict__ v, int nb)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        int64_t run = 0;
-        for (int i = 0; i < nb; i++) {
-            const int64_t t = v[i];
-            v[i] = run;
-            run += t;
+    __shared__ int64_t part[32];
+    __shared__ int64_t carry;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0)
+        carry = 0;
+    __syncthreads();
+    for (int base = 0; base < nb; base += 1024) {
+        const int i = base + threadIdx.x;
+        const int64_t own = i < nb ? v[i] : 0;
+        int64_t s = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t t = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o)
+                s += t;
         }
-        v[nb] = run;
+        if (lane == 31)
+            part[warp] = s;
+        __syncthreads();
+        if (warp == 0) {
+            const int64_t p = part[lane];
+            int64_t q = p;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int64_t t = __shfl_up_sync(0xffffffffu, q, o);
+                if (lane >= o)
+                    q += t;
+            }
+            part[lane] = q - p;
+        }
+        __syncthreads();
+        const int64_t before = carry + part[warp] + s - own;
+        if (i < nb)
+            v[i] = before;
+        __syncthreads();
+        if (threadIdx.x == 1023)
+            carry = before + own;
+        __syncthreads();
     }
+    if (threadIdx.x == 0)
+        v[nb] = carry;
 }
 
 __global__ void finish_ptr_kernel(int64_t* __restrict__ ptr, int n, const int32_t* __restrict__ len)
@@ -669,7 +703,7 @@ cudaError_t launch_scan_lengths(const int32_t* len, int n, int64_t* ptr, int64_t
     const int bs = 1024;
     const int nb = (n + bs - 1) / bs;
     scan_blocks_kernel<<<nb, bs, 0, st>>>(len, n, ptr, tmp);
-    scan_serial_kernel<<<1, 1, 0, st>>>(tmp, nb);
+    scan_sums_kernel<<<1, 1024, 0, st>>>(tmp, nb);
     scan_add_kernel<<<nb, bs, 0, st>>>(ptr, n, tmp);
     finish_ptr_kernel<<<1, 1, 0, st>>>(ptr, n, len);
     return cudaGetLastError();
