@@ -410,9 +410,6 @@ __global__ void __launch_bounds__(256)
         }
         int row = e < e1 ? __ldg(pb.cidx + e) : 0x7fffffff;
         double val = e < e1 ? __ldg(pb.cval + e) : 0.0;
-        // the entry after it, on its way while a row is worked on
-        int next_row = e + 1 < e1 ? __ldg(pb.cidx + e + 1) : 0x7fffffff;
-        double next_val = e + 1 < e1 ? __ldg(pb.cval + e + 1) : 0.0;
         int brow = q < q1 ? __ldg(pb.bidx + q) : 0x7fffffff;
         double loss = 0.0;
         bool seen = pb.bptr != nullptr || col < 0;  // identity target: e_col met in I_k
@@ -461,10 +458,8 @@ __global__ void __launch_bounds__(256)
             if (mine) {
                 atomicAdd(&io.dC[e], -(r * x) * (2.0 * io.wres));
                 e++;
-                row = next_row;
-                val = next_val;
-                next_row = e + 1 < e1 ? __ldg(pb.cidx + e + 1) : 0x7fffffff;
-                next_val = e + 1 < e1 ? __ldg(pb.cval + e + 1) : 0.0;
+                row = e < e1 ? __ldg(pb.cidx + e) : 0x7fffffff;
+                val = e < e1 ? __ldg(pb.cval + e) : 0.0;
             }
         }
         outside(0x7fffffff);

@@ -24,8 +24,8 @@
 //   Bound: latency of the blocked Cholesky and of the triangular solves at two
 //   CTAs of 256 threads per SM (mixed), one (FP64).  8,000 block columns of a
 //   20^3 27-point stencil with 3 x 3 blocks: 36.9 ms in the general solver, 12.7 ms
-//   here; 64,000 of the block diagonal (3 unknowns, 246 entries, CTAs of 64
-//   threads): 3.6 ms there, 2.7 ms here.
+//   here; 64,000 of the block diagonal (3 unknowns, 246 entries, eight lanes
+//   each; CTAs of 64 threads took 2.7): 3.6 ms there, 1.7 ms here.
 #include "fixed_solve.cuh"
 #include "spai_kernels.h"
 
@@ -398,9 +398,6 @@ __global__ void __launch_bounds__(128)
             int64_t e = a0, q = q0;
             int row = e < a1 ? __ldg(pb.cidx + e) : 0x7fffffff;
             double val = e < a1 ? __ldg(pb.cval + e) : 0.0;
-            // the entry after it, on its way while a row is worked on
-            int next_row = e + 1 < a1 ? __ldg(pb.cidx + e + 1) : 0x7fffffff;
-            double next_val = e + 1 < a1 ? __ldg(pb.cval + e + 1) : 0.0;
             int brow = pb.bptr ? (q < q1 ? __ldg(pb.bidx + q) : 0x7fffffff)
                                : (kb >= 0 && l8 < bs ? bs * kb + l8 : 0x7fffffff);
             double part = 0.0;
@@ -441,10 +438,8 @@ __global__ void __launch_bounds__(128)
                 }
                 if (mine) {
                     e++;
-                    row = next_row;
-                    val = next_val;
-                    next_row = e + 1 < a1 ? __ldg(pb.cidx + e + 1) : 0x7fffffff;
-                    next_val = e + 1 < a1 ? __ldg(pb.cval + e + 1) : 0.0;
+                    row = e < a1 ? __ldg(pb.cidx + e) : 0x7fffffff;
+                    val = e < a1 ? __ldg(pb.cval + e) : 0.0;
                 }
             }
             r2 = part;
