@@ -831,16 +831,33 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             use_warp && (adaptive || mspai::warp_slot_bytes(cap, elem_b) *
                                              (mspai::kWarpKernelThreads / 32) > 200 * 1024);
         if (warp_global) {
-            const size_t need = mspai::warp_global_scratch_bytes(cap, elem_b, count);
-            CUDA_TRY(h, h->scratch.ensure(need));
-            if (adaptive)  // the candidate bit vectors of the slots start cleared
-                CUDA_TRY(h, cudaMemsetAsync(h->scratch.p, 0, need, st));
             if (nsmall == 0)
                 CUDA_TRY(h, cudaEventRecord(h->evb[0], st));
-            h->launches++;
-            CUDA_TRY(h, mspai::launch_warp_solve_global(elem_b, pbb, cap, out, list, count,
-                                                        counter, h->scratch.as<char>(),
-                                                        h->scratch.bytes, st, &grid));
+            // adaptive columns first in shared memory: what outgrows the slots
+            // there starts again below
+            if (adaptive && elem_b == 8 && pbb.refine == 0 && !out.rstore &&
+                pbb.mn <= mspai::kShareMn) {
+                int32_t* rest = h->lists.as<int32_t>() + static_cast<size_t>(kLists) * nprob;
+                CUDA_TRY(h, cudaMemsetAsync(dcnt + 28, 0, sizeof(int32_t), st));
+                h->launches++;
+                CUDA_TRY(h, mspai::launch_warp_adaptive(pbb, out, list, count, counter, rest,
+                                                        dcnt + 28, st));
+                CUDA_TRY(h, cudaMemcpyAsync(&left, dcnt + 28, sizeof(int32_t),
+                                            cudaMemcpyDeviceToHost, st));
+                CUDA_TRY(h, cudaStreamSynchronize(st));
+                CUDA_TRY(h, cudaMemsetAsync(counter, 0, sizeof(int32_t), st));
+                list = rest;
+            }
+            if (left > 0) {
+                const size_t need = mspai::warp_global_scratch_bytes(cap, elem_b, left);
+                CUDA_TRY(h, h->scratch.ensure(need));
+                if (adaptive)  // the candidate bit vectors of the slots start cleared
+                    CUDA_TRY(h, cudaMemsetAsync(h->scratch.p, 0, need, st));
+                h->launches++;
+                CUDA_TRY(h, mspai::launch_warp_solve_global(elem_b, pbb, cap, out, list, left,
+                                                            counter, h->scratch.as<char>(),
+                                                            h->scratch.bytes, st, &grid));
+            }
             CUDA_TRY(h, cudaEventRecord(h->evb[1], st));
             timed[0] = true;
             h->stats.bucket_columns[0] = count + nsmall;

@@ -173,6 +173,8 @@ __global__ void __launch_bounds__(kWarpKernelThreads)
     const int w = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     WarpGroup g{&sc[w]};
+    pb.bs = 1;  // scalar columns only: the block code and its local arrays go
+    pb.qru = 0;
     SlotLayout<T> lay(cap, false);
     Slot<T> s = lay.at(smem + static_cast<size_t>(w) * slot_bytes, nullptr);
     while (true) {
@@ -199,6 +201,8 @@ __global__ void __launch_bounds__(kWarpKernelThreads)
     const int w = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     WarpGroup g{&sc[w]};
+    pb.bs = 1;  // scalar columns only: the block code and its local arrays go
+    pb.qru = 0;
     SlotLayout<T> lay(cap, false);
     const size_t slot_id = static_cast<size_t>(blockIdx.x) * (kWarpKernelThreads / 32) + w;
     Slot<T> s = lay.at(scratch + slot_id * slot_bytes, nullptr);
@@ -210,6 +214,92 @@ __global__ void __launch_bounds__(kWarpKernelThreads)
         if (t >= count)
             break;
         solve_column<T>(g, pb, cap, s, out, list[t]);
+    }
+}
+
+// The same with the whole slot in shared memory, for adaptive scalar columns
+// that end within kShareN unknowns and kShareE entries (FP64, no refinement);
+// a column that outgrows it is appended to rest and starts again in the kernel
+// above.  The arrays of the pattern update take W's place, which is dead by
+// then; the candidates are collected in a hash set instead of a bit vector.
+//   Bound: latency, 16 warps per SM (registers; the slots take 91 KB per CTA of
+//   eight).
+constexpr int kShareN = 16;
+constexpr int kShareE = 112;      // 16 columns of a 7-point stencil
+constexpr int kShareMw = 44;      // rows of the folded matrix
+constexpr int kShareCand = 192;   // unique candidates
+
+struct ShareSlot {
+    uint64_t keys[kShareE];
+    double ev[kShareE], r[kShareE], x[kShareN], gv[kShareN];
+    union {
+        double W[kShareMw * (kShareN + 1)];
+        struct {
+            double rho[kShareCand];
+            int32_t cand[256];  // next_pow2(kShareCand)
+            int32_t ctmp[kShareCand + 1];
+            int32_t ctab[kCandTable];
+        } u;
+    };
+    int32_t J[kShareN + kShareMn], off[kShareN + 1], ejj[kShareE], pos[kShareE + 1], I[kShareE],
+        rstart[kShareE + 1], tmp[kShareE + 1];
+};
+
+__global__ void __launch_bounds__(kWarpKernelThreads, 2)
+    warp_adaptive_kernel(Problem pb, Output out, const int32_t* __restrict__ list, int count,
+                         int32_t* __restrict__ counter, int32_t* __restrict__ rest,
+                         int32_t* __restrict__ rest_count)
+{
+    // constants here: the solver's other branches go
+    pb.bs = 1;
+    pb.qru = 0;
+    pb.refine = 0;
+    out.rstore = nullptr;
+    Caps cap{};
+    cap.emax = kShareE;
+    cap.nmax = kShareN;
+    cap.mwmax = kShareMw;
+    cap.cmax = kShareCand;
+    cap.nrhs = 1;
+    extern __shared__ __align__(16) char smem[];
+    __shared__ GroupScratch sc[kWarpKernelThreads / 32];
+    const int w = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    WarpGroup g{&sc[w]};
+    ShareSlot& a = reinterpret_cast<ShareSlot*>(smem)[w];
+    Slot<double> s{};
+    s.J = a.J;
+    s.off = a.off;
+    s.ejj = a.ejj;
+    s.ev = a.ev;
+    s.pos = a.pos;
+    s.keys = a.keys;
+    s.I = a.I;
+    s.rstart = a.rstart;
+    s.tmp = a.tmp;
+    s.r = a.r;
+    s.W = s.Wfast = a.W;
+    s.wfast_elems = kShareMw * (kShareN + 1);
+    s.x = a.x;
+    s.gv = a.gv;
+    s.cand = a.u.cand;
+    s.ctmp = a.u.ctmp;
+    s.rho = a.u.rho;
+    s.ctab = a.u.ctab;
+    while (true) {
+        int t = 0;
+        if (lane == 0)
+            t = atomicAdd(counter, 1);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >= count)
+            break;
+        const int col = list[t];
+        solve_column<double>(g, pb, cap, s, out, col);
+        if (lane == 0 && out.status[col] == 3) {
+            for (int q = 0; q < 3; q++)
+                out.work[3 * static_cast<size_t>(col) + q] = 0.0;
+            rest[atomicAdd(rest_count, 1)] = col;
+        }
     }
 }
 
@@ -607,6 +697,28 @@ cudaError_t launch_warp_solve_global(int elem_bytes, const Problem& pb, const Ca
                                            scratch_bytes, st, grid_out);
     return launch_warp_global_t<double>(pb, cap, out, list, count, counter, scratch,
                                         scratch_bytes, st, grid_out);
+}
+
+cudaError_t launch_warp_adaptive(const Problem& pb, const Output& out, const int32_t* list,
+                                 int count, int32_t* counter, int32_t* rest,
+                                 int32_t* rest_count, cudaStream_t st)
+{
+    const size_t smem = sizeof(ShareSlot) * (kWarpKernelThreads / 32);
+    cudaError_t e = cudaFuncSetAttribute(warp_adaptive_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem));
+    if (e != cudaSuccess)
+        return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, warp_adaptive_kernel,
+                                                      kWarpKernelThreads, smem);
+    if (e != cudaSuccess)
+        return e;
+    const int need = (count + kWarpKernelThreads / 32 - 1) / (kWarpKernelThreads / 32);
+    const int grid = std::max(1, std::min(std::max(per_sm, 1) * num_sms(), need));
+    warp_adaptive_kernel<<<grid, kWarpKernelThreads, smem, st>>>(pb, out, list, count, counter,
+                                                                 rest, rest_count);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_warp_solve(int elem_bytes, const Problem& pb, const Caps& cap,

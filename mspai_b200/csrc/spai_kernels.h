@@ -72,6 +72,14 @@ size_t w_bytes(const Caps& cap, int elem_bytes);
 // CTAs per SM of the solver for this element size and shared-memory area
 int cta_per_sm(int elem_bytes, size_t smem_w_bytes);
 size_t cta_scratch_needed(int elem_bytes, const Caps& cap, int count, size_t smem_w_bytes);
+
+// adaptive scalar columns, FP64 without refinement, at most kShareMn unknowns
+// added in an update: the slots in shared memory; the columns that outgrow them
+// to rest (*rest_count starts at zero)
+constexpr int kShareMn = 16;
+cudaError_t launch_warp_adaptive(const Problem& pb, const Output& out, const int32_t* list,
+                                 int count, int32_t* counter, int32_t* rest,
+                                 int32_t* rest_count, cudaStream_t st);
 cudaError_t launch_warp_solve(int elem_bytes, const Problem& pb, const Caps& cap,
                               const Output& out, const int32_t* list, int count, int32_t* counter,
                               cudaStream_t st, int* grid_out);

@@ -34,6 +34,9 @@ namespace mspai {
 
 
 
+constexpr int kCandTableBits = 9;
+constexpr int kCandTable = 1 << kCandTableBits;
+
 // Read-only inputs of a setup (device pointers).
 struct Problem {
     int n;                                   // columns of C and M
@@ -128,6 +131,7 @@ struct Slot {
     int32_t* cand;     // lcand candidate column indices (adaptive)
     int32_t* ctmp;     // cmax + 1 candidate flags / scan
     uint32_t* bmap;    // nbmap words: bit vector over problem columns (adaptive)
+    int32_t* ctab;     // kCandTable words: hash set in its place (slots in shared memory)
     double* rho;       // cmax
 };
 
@@ -231,6 +235,7 @@ struct SlotLayout {
             s.W = reinterpret_cast<T*>(base + o_W);
         }
         s.rhs = nullptr;  // set by the caller from mw
+        s.ctab = nullptr;
         s.Wfast = nullptr;
         s.wfast_elems = 0;
         s.bsc = nullptr;
@@ -299,16 +304,54 @@ __device__ void group_householder(const G& g, T* W, int ld, int mw, int n, int n
             wk[i] *= scale;
         g.sync();
         // apply H = I - tau v v^T (v_k = 1) to the later columns and the rhs
-        for (int c = k + 1 + g.warp(); c < n + nrhs; c += G::kWarps) {
-            T* col = W + static_cast<size_t>(c) * ld;
-            T d = (lane == 0) ? col[k] : T(0);
-            for (int i = k + 1 + lane; i < mw; i += 32)
-                d += wk[i] * col[i];
-            d = warp_sum(d) * tau;
-            if (lane == 0)
-                col[k] -= d;
-            for (int i = k + 1 + lane; i < mw; i += 32)
-                col[i] -= d * wk[i];
+        if constexpr (G::kWarps == 1) {
+            // four columns at a time: their shuffle chains overlap (the sums of
+            // a column are those of the loop below)
+            for (int c0 = k + 1; c0 < n + nrhs; c0 += 4) {
+                T* col[4];
+                T d[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    col[q] = W + static_cast<size_t>(min(c0 + q, n + nrhs - 1)) * ld;
+                    d[q] = (lane == 0) ? col[q][k] : T(0);
+                }
+                for (int i = k + 1 + lane; i < mw; i += 32) {
+                    const T v = wk[i];
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        d[q] += v * col[q][i];
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int q = 0; q < 4; q++)
+                        d[q] += __shfl_xor_sync(0xffffffffu, d[q], o);
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    d[q] *= tau;
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    if (c0 + q >= n + nrhs)
+                        break;
+                    if (lane == 0)
+                        col[q][k] -= d[q];
+                    for (int i = k + 1 + lane; i < mw; i += 32)
+                        col[q][i] -= d[q] * wk[i];
+                }
+            }
+        }
+        else {
+            for (int c = k + 1 + g.warp(); c < n + nrhs; c += G::kWarps) {
+                T* col = W + static_cast<size_t>(c) * ld;
+                T d = (lane == 0) ? col[k] : T(0);
+                for (int i = k + 1 + lane; i < mw; i += 32)
+                    d += wk[i] * col[i];
+                d = warp_sum(d) * tau;
+                if (lane == 0)
+                    col[k] -= d;
+                for (int i = k + 1 + lane; i < mw; i += 32)
+                    col[i] -= d * wk[i];
+            }
         }
         g.sync();
     }
@@ -732,7 +775,53 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
         const bool merge = s.Wfast && E > 0 &&
                            merge_bytes <= static_cast<size_t>(s.wfast_elems) * sizeof(T);
         uint64_t* kdst = merge ? reinterpret_cast<uint64_t*>(s.Wfast) : s.keys;
-        for (int jj = g.warp(); jj < n; jj += G::kWarps) {
+        int longest = 0;  // entries of a column (a warp's columns only)
+        if constexpr (G::kWarps == 1) {
+            // eight lanes a column, eight columns' first entries in flight
+            const int grp = lane >> 3, l8 = lane & 7;
+            for (int c0 = 0; c0 < n; c0 += 32) {
+                const int cn = min(32, n - c0);
+                int64_t b0 = 0;
+                int o0 = 0, len0 = 0;
+                if (lane < cn) {
+                    b0 = __ldg(pb.cptr + scol(c0 + lane));
+                    o0 = s.off[c0 + lane];
+                    len0 = s.off[c0 + lane + 1] - o0;
+                }
+                longest = max(longest, __reduce_max_sync(0xffffffffu, len0));
+                for (int q = 0; q < cn; q += 8) {
+                    int64_t b[2];
+                    int o[2], len[2], row[2] = {0, 0};
+                    double v[2] = {0.0, 0.0};
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int src = q + 4 * h + grp;
+                        b[h] = __shfl_sync(0xffffffffu, b0, src);
+                        o[h] = __shfl_sync(0xffffffffu, o0, src);
+                        len[h] = __shfl_sync(0xffffffffu, len0, src);
+                        if (l8 < len[h]) {
+                            row[h] = __ldg(pb.cidx + b[h] + l8);
+                            v[h] = __ldg(pb.cval + b[h] + l8);
+                        }
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        for (int t = l8; t < len[h]; t += 8) {
+                            const int e = o[h] + t;
+                            if (t != l8) {
+                                row[h] = __ldg(pb.cidx + b[h] + t);
+                                v[h] = __ldg(pb.cval + b[h] + t);
+                            }
+                            s.ejj[e] = c0 + q + 4 * h + grp;
+                            s.ev[e] = v[h];
+                            kdst[e] = (static_cast<uint64_t>(row[h]) << kEntryBits) |
+                                      static_cast<uint64_t>(e);
+                        }
+                    }
+                }
+            }
+        }
+        for (int jj = g.warp(); G::kWarps > 1 && jj < n; jj += G::kWarps) {
             const int j = scol(jj);
             const int64_t base = pb.cptr[j];
             const int o = s.off[jj];
@@ -883,8 +972,40 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                     }
                 }
             }
-            // singleton rows, folded per column (one warp per column)
-            for (int jj = g.warp(); jj < n; jj += G::kWarps) {
+            // singleton rows, folded per column (one warp per column; columns of
+            // at most eight entries by eight lanes each: the same sums, the other
+            // 24 lanes would add zeros)
+            bool folded = false;
+            if constexpr (G::kWarps == 1) {
+                folded = nrhs == 1 && longest <= 8 && !structured;
+                for (int j0 = 0; folded && j0 < n; j0 += 4) {
+                    const int jj = j0 + (lane >> 3);
+                    const int e = jj < n ? s.off[jj] + (lane & 7) : 0;
+                    double sig = 0.0, tb = 0.0;
+                    if (jj < n && e < s.off[jj + 1]) {
+                        int u = 0;
+                        const bool single =
+                            fixed ? s.pos[e] < 0
+                                  : (u = s.pos[e], s.rstart[u + 1] - s.rstart[u] == 1);
+                        if (single) {
+                            const double v = s.ev[e];
+                            sig = v * v;
+                            tb = v * (fixed ? s.r[e] : target_value(pb, col, s.I[u]));
+                        }
+                    }
+#pragma unroll
+                    for (int o = 4; o > 0; o >>= 1) {
+                        sig += __shfl_xor_sync(0xffffffffu, sig, o);
+                        tb += __shfl_xor_sync(0xffffffffu, tb, o);
+                    }
+                    if (jj < n && (lane & 7) == 0) {
+                        const double nrm = sqrt(sig);
+                        W[static_cast<size_t>(jj) * ld + S + jj] = static_cast<T>(nrm);
+                        rhs[S + jj] = static_cast<T>(nrm > 0.0 ? tb / nrm : 0.0);
+                    }
+                }
+            }
+            for (int jj = g.warp(); !folded && jj < n; jj += G::kWarps) {
                 double sig = 0.0;
                 double tb[kMaxBlockSize] = {};
                 for (int e = s.off[jj] + lane; e < s.off[jj + 1]; e += 32) {
@@ -1176,7 +1297,65 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
         if (g.rank() == 0)
             g.sc->i[1] = 0;
         g.sync();
-        for (int u = g.warp(); u < nl; u += G::kWarps) {
+        // slots in shared memory: a hash set of kCandTable columns instead of the
+        // bit vector (its atomics went to the L2), eight lanes a row, eight rows'
+        // first entries in flight.  More columns than the list holds: status 3
+        // below, and the caller gives the column to a larger slot.
+        bool hashed = false;
+        if constexpr (G::kWarps == 1) {
+            hashed = s.ctab != nullptr;
+            if (hashed) {
+                for (int i = lane; i < kCandTable; i += 32)
+                    s.ctab[i] = -1;
+                __syncwarp();
+            }
+            const int grp = lane >> 3, l8 = lane & 7;
+            auto insert = [&](int c) {
+                uint32_t h = (static_cast<uint32_t>(c) * 2654435761u) >> (32 - kCandTableBits);
+                for (int probe = 0; probe < kCandTable; probe++) {
+                    const int old = atomicCAS(&s.ctab[h], -1, c);
+                    if (old == c)
+                        return;
+                    if (old == -1) {
+                        const int idx = atomicAdd(&g.sc->i[1], 1);
+                        if (idx < cap.cmax)
+                            s.cand[idx] = c;
+                        return;
+                    }
+                    h = (h + 1) & (kCandTable - 1);
+                }
+                atomicAdd(&g.sc->i[1], cap.cmax + 1);  // the table is full
+            };
+            for (int u0 = 0; hashed && u0 < nl; u0 += 32) {
+                const int un = min(32, nl - u0);
+                int64_t b0 = 0;
+                int len0 = 0;
+                if (lane < un) {
+                    const int l = u0 + lane < m ? lrows[u0 + lane] : s.pos[0];
+                    if (l < pb.n) {
+                        b0 = __ldg(pb.rptr + l);
+                        len0 = static_cast<int>(__ldg(pb.rptr + l + 1) - b0);
+                    }
+                }
+                for (int q = 0; q < un; q += 8) {
+                    int64_t b[2];
+                    int len[2], c[2] = {0, 0};
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const int src = q + 4 * h + grp;
+                        b[h] = __shfl_sync(0xffffffffu, b0, src);
+                        len[h] = __shfl_sync(0xffffffffu, len0, src);
+                        if (l8 < len[h])
+                            c[h] = __ldg(pb.rcol + b[h] + l8);
+                    }
+#pragma unroll
+                    for (int h = 0; h < 2; h++)
+                        for (int t = l8; t < len[h]; t += 8)
+                            insert(t == l8 ? c[h] : __ldg(pb.rcol + b[h] + t));
+                }
+            }
+        }
+        for (int u = g.warp(); !hashed && u < nl; u += G::kWarps) {
             int r0, r1;
             if (bs == 1) {
                 const int l = (u < m) ? lrows[u] : s.pos[0];
@@ -1207,7 +1386,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
         const int nu = g.sc->i[1];
         const int T_c = min(nu, cap.cmax);
         // clear the bit vector for the next use (every set bit is listed)
-        for (int t = g.rank(); t < T_c; t += G::kSize)
+        for (int t = g.rank(); !hashed && t < T_c; t += G::kSize)
             s.bmap[s.cand[t] >> 5] = 0u;
         g.sync();
         if (nu > cap.cmax) {
@@ -1258,12 +1437,24 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
             const int j = s.cand[t];
             if (bs == 1) {
                 double a2 = 0.0, num = 0.0;
-                for (int64_t p = pb.cptr[j]; p < pb.cptr[j + 1]; p++) {
-                    const double v = pb.cval[p];
-                    a2 += v * v;
-                    const int u = lower_bound_i32(s.I, m, pb.cidx[p]);
-                    if (u < m && s.I[u] == pb.cidx[p])
-                        num += s.r[u] * v;
+                const int64_t pe = pb.cptr[j + 1];
+                for (int64_t p = pb.cptr[j]; p < pe; p += 4) {  // four entries in flight
+                    int row[4];
+                    double v[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        row[q] = p + q < pe ? __ldg(pb.cidx + p + q) : -1;
+                        v[q] = p + q < pe ? __ldg(pb.cval + p + q) : 0.0;
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        if (row[q] < 0)
+                            break;
+                        a2 += v[q] * v[q];
+                        const int u = lower_bound_i32(s.I, m, row[q]);
+                        if (u < m && s.I[u] == row[q])
+                            num += s.r[u] * v[q];
+                    }
                 }
                 const double ajn = sqrt(a2);
                 s.rho[t] = sqrt(res2 - (num * num) / (ajn * ajn));
