@@ -245,31 +245,60 @@ __device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Prob
     // ---- r = b - C x per right-hand side, its squared norm; with grad C^T r
     auto residual = [&](bool grad) -> double {
         double part = 0.0;
-        for (int t = tid; t < m * bs; t += NT) {
-            const int c = t / m, u = t - c * m;
-            double v = target_value(pb, bs * kb + c, I[u]);
-            const double* xc = x + c * n;
-            for (int q = rs[u]; q < rs[u + 1]; q++)
-                v -= value(by[q], bj[q]) * xc[bj[q]];
-            r[t] = v;
-            part += v * v;
+        // all right-hand sides of a row by one thread: its values are read once
+        for (int u = tid; u < m; u += NT) {
+            double v[kMaxBlockSize];
+#pragma unroll
+            for (int c = 0; c < kMaxBlockSize; c++)
+                v[c] = c < bs ? target_value(pb, bs * kb + c, I[u]) : 0.0;
+            const int q1 = rs[u + 1];
+#pragma unroll 4
+            for (int q = rs[u]; q < q1; q++) {
+                const int jj = bj[q];
+                const double a = value(by[q], jj);
+#pragma unroll
+                for (int c = 0; c < kMaxBlockSize; c++)
+                    if (c < bs)
+                        v[c] -= a * x[c * n + jj];
+            }
+#pragma unroll
+            for (int c = 0; c < kMaxBlockSize; c++)
+                if (c < bs) {
+                    r[c * m + u] = v[c];
+                    part += v[c] * v[c];
+                }
         }
         const double r2 = g.sum(part);  // includes a barrier: r is complete
         if (grad) {
             // eight lanes per column (warp-uniform trips)
-            for (int t0 = 0; t0 < n * bs; t0 += NT / 8) {
-                const int t = t0 + tid / 8, q = tid & 7;
-                double acc = 0.0;
-                if (t < n * bs) {
-                    const int c = t / n, jj = t - c * n;
-                    for (int e = off[jj] + q; e < off[jj + 1]; e += 8)
-                        acc += value(e, jj) * r[c * m + R[e]];
+            for (int j0 = 0; j0 < n; j0 += NT / 8) {
+                const int jj = j0 + tid / 8, q = tid & 7;
+                double acc[kMaxBlockSize];
+#pragma unroll
+                for (int c = 0; c < kMaxBlockSize; c++)
+                    acc[c] = 0.0;
+                if (jj < n) {
+                    const int e1 = off[jj + 1];
+#pragma unroll 4
+                    for (int e = off[jj] + q; e < e1; e += 8) {
+                        const double a = value(e, jj);
+                        const double* re = r + R[e];
+#pragma unroll
+                        for (int c = 0; c < kMaxBlockSize; c++)
+                            if (c < bs)
+                                acc[c] += a * re[c * m];
+                    }
                 }
-                acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-                acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-                acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-                if (t < n * bs && q == 0)
-                    gv[t] = static_cast<T>(acc);
+#pragma unroll
+                for (int c = 0; c < kMaxBlockSize; c++) {
+                    if (c >= bs)
+                        break;
+                    acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 4);
+                    acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 2);
+                    acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 1);
+                    if (jj < n && q == 0)
+                        gv[c * n + jj] = static_cast<T>(acc[c]);
+                }
             }
             g.sync();
         }
