@@ -69,24 +69,8 @@ __global__ void csr_gather_kernel(const int64_t* __restrict__ tptr, const int32_
     const int warps = (gridDim.x * blockDim.x) >> 5;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nrows; i += warps) {
         double s = 0.0;
-        const int64_t end = tptr[i + 1];
-        for (int64_t t = tptr[i] + lane; t < end; t += 128) {
-            int c[4];
-            double v[4], xc[4];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const bool in = t + 32 * q < end;
-                c[q] = in ? __ldcs(tcol + t + 32 * q) : -1;
-                v[q] = in ? __ldcs(tval + t + 32 * q) : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                xc[q] = c[q] >= 0 ? __ldg(x + c[q]) : 0.0;
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (c[q] >= 0)
-                    s += v[q] * xc[q];
-        }
+        for (int64_t t = tptr[i] + lane; t < tptr[i + 1]; t += 32)
+            s += tval[t] * x[tcol[t]];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
             s += __shfl_xor_sync(0xffffffffu, s, o);
