@@ -10,6 +10,12 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+// Before a loop that a warp's column passes a few times only: the warp kernels'
+// file keeps these rolled (spai_warp.cu), elsewhere the compiler decides.
+#ifndef MSPAI_LOOP
+#define MSPAI_LOOP
+#endif
+
 namespace mspai {
 
 // Optional per-phase cycle counters (profiling builds only: -DMSPAI_PHASE_TIMERS).
@@ -215,8 +221,11 @@ __device__ int group_exclusive_scan(const G& g, int* a, int len)
 template <class G, class K>
 __device__ void group_bitonic_sort(const G& g, K* keys, int L)
 {
+MSPAI_LOOP
     for (int k = 2; k <= L; k <<= 1) {
+MSPAI_LOOP
         for (int j = k >> 1; j > 0; j >>= 1) {
+MSPAI_LOOP
             for (int i = g.rank(); i < L; i += G::kSize) {
                 const int ixj = i ^ j;
                 if (ixj > i) {
@@ -245,6 +254,7 @@ template <class K, class G>
 __device__ K* group_merge_runs(const G& g, K* a, K* b, int E, const int* off, int n)
 {
     const int chunk = (E + G::kSize - 1) / G::kSize;
+MSPAI_LOOP
     for (int w = 1; w < n; w <<= 1) {
         const int npairs = (n + 2 * w - 1) / (2 * w);
         int o = min(E, g.rank() * chunk);
@@ -252,6 +262,7 @@ __device__ K* group_merge_runs(const G& g, K* a, K* b, int E, const int* off, in
         while (o < oe) {
             // the last pair whose output starts at or before o
             int lo = 0, hi = npairs - 1;
+MSPAI_LOOP
             while (lo < hi) {
                 const int mid = (lo + hi + 1) >> 1;
                 if (off[min(2 * mid * w, n)] <= o)
@@ -265,6 +276,7 @@ __device__ K* group_merge_runs(const G& g, K* a, K* b, int E, const int* off, in
             const int la = s1 - s0, lb = s2 - s1, d = o - s0;
             // keys of the first half among the pair's first d outputs
             int ilo = max(0, d - lb), ihi = min(d, la);
+MSPAI_LOOP
             while (ilo < ihi) {
                 const int i = (ilo + ihi) >> 1;
                 if (a[s0 + i] <= a[s1 + d - i - 1])
@@ -274,6 +286,7 @@ __device__ K* group_merge_runs(const G& g, K* a, K* b, int E, const int* off, in
             }
             int ia = s0 + ilo, ib = s1 + (d - ilo);
             const int end = min(oe, s2);
+MSPAI_LOOP
             for (; o < end; o++) {
                 const bool take_a = ib >= s2 || (ia < s1 && a[ia] <= a[ib]);
                 b[o] = take_a ? a[ia++] : a[ib++];

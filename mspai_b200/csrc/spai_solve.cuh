@@ -265,6 +265,7 @@ __device__ __forceinline__ double target_value(const Problem& pb, int col, int r
 __device__ __forceinline__ int lower_bound_i32(const int32_t* a, int len, int v)
 {
     int lo = 0, hi = len;
+    MSPAI_LOOP
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
         if (a[mid] < v)
@@ -288,6 +289,7 @@ __device__ void group_householder(const G& g, T* W, int ld, int mw, int n, int n
     for (int k = 0; k < kmax; k++) {
         T* wk = W + static_cast<size_t>(k) * ld;
         T part = 0;
+MSPAI_LOOP
         for (int i = k + 1 + g.rank(); i < mw; i += G::kSize)
             part += wk[i] * wk[i];
         const T xnorm2 = g.sum(part);
@@ -300,6 +302,7 @@ __device__ void group_householder(const G& g, T* W, int ld, int mw, int n, int n
         g.sync();
         if (g.rank() == 0)
             wk[k] = beta;
+MSPAI_LOOP
         for (int i = k + 1 + g.rank(); i < mw; i += G::kSize)
             wk[i] *= scale;
         g.sync();
@@ -307,6 +310,7 @@ __device__ void group_householder(const G& g, T* W, int ld, int mw, int n, int n
         if constexpr (G::kWarps == 1) {
             // four columns at a time: their shuffle chains overlap (the sums of
             // a column are those of the loop below)
+#pragma unroll 1
             for (int c0 = k + 1; c0 < n + nrhs; c0 += 4) {
                 T* col[4];
                 T d[4];
@@ -315,6 +319,7 @@ __device__ void group_householder(const G& g, T* W, int ld, int mw, int n, int n
                     col[q] = W + static_cast<size_t>(min(c0 + q, n + nrhs - 1)) * ld;
                     d[q] = (lane == 0) ? col[q][k] : T(0);
                 }
+MSPAI_LOOP
                 for (int i = k + 1 + lane; i < mw; i += 32) {
                     const T v = wk[i];
 #pragma unroll
@@ -335,20 +340,24 @@ __device__ void group_householder(const G& g, T* W, int ld, int mw, int n, int n
                         break;
                     if (lane == 0)
                         col[q][k] -= d[q];
+MSPAI_LOOP
                     for (int i = k + 1 + lane; i < mw; i += 32)
                         col[q][i] -= d[q] * wk[i];
                 }
             }
         }
         else {
+MSPAI_LOOP
             for (int c = k + 1 + g.warp(); c < n + nrhs; c += G::kWarps) {
                 T* col = W + static_cast<size_t>(c) * ld;
                 T d = (lane == 0) ? col[k] : T(0);
+MSPAI_LOOP
                 for (int i = k + 1 + lane; i < mw; i += 32)
                     d += wk[i] * col[i];
                 d = warp_sum(d) * tau;
                 if (lane == 0)
                     col[k] -= d;
+MSPAI_LOOP
                 for (int i = k + 1 + lane; i < mw; i += 32)
                     col[i] -= d * wk[i];
             }
@@ -364,6 +373,7 @@ template <class T, class G>
 __device__ int group_back_substitute(const G& g, const T* W, int ld, int n, T* rhs, double* x)
 {
     int singular = 0;
+MSPAI_LOOP
     for (int j = g.rank(); j < n; j += G::kSize)
         if (W[static_cast<size_t>(j) * ld + j] == T(0))
             singular = 1;
@@ -376,12 +386,14 @@ __device__ int group_back_substitute(const G& g, const T* W, int ld, int n, T* r
             if (lane == 0)
                 rhs[j] = xj;
             const T* wj = W + static_cast<size_t>(j) * ld;
+MSPAI_LOOP
             for (int i = lane; i < j; i += 32)
                 rhs[i] -= wj[i] * xj;
             __syncwarp();
         }
     }
     g.sync();
+MSPAI_LOOP
     for (int j = g.rank(); j < n; j += G::kSize)
         x[j] = static_cast<double>(rhs[j]);
     g.sync();
@@ -432,6 +444,7 @@ __device__ double group_residual(const G& g, const Problem& pb, int col, const u
                                  int nrhs)
 {
     double part = 0.0;
+MSPAI_LOOP
     for (int t = g.rank(); t < m * nrhs; t += G::kSize) {
         const int c = t / m, u = t - c * m;
         double v = target_value(pb, pb.bs * col + c, I[u]);
@@ -739,6 +752,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
         status = 3;
         nbk = 0;
     }
+MSPAI_LOOP
     for (int t = g.rank(); t < nbk; t += G::kSize)
         s.J[t] = pb.pidx[p0 + t];
     g.sync();
@@ -754,6 +768,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
     for (int step = -1; step < pb.ns && status != 3; step++) {
         n = nbk * bs;
         // ---- 1. entries of C(:, J), sorted by row
+MSPAI_LOOP
         for (int jj = g.rank(); jj < n; jj += G::kSize) {
             const int j = scol(jj);
             s.off[jj] = static_cast<int>(pb.cptr[j + 1] - pb.cptr[j]);
@@ -779,6 +794,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
         if constexpr (G::kWarps == 1) {
             // eight lanes a column, eight columns' first entries in flight
             const int grp = lane >> 3, l8 = lane & 7;
+MSPAI_LOOP
             for (int c0 = 0; c0 < n; c0 += 32) {
                 const int cn = min(32, n - c0);
                 int64_t b0 = 0;
@@ -789,6 +805,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                     len0 = s.off[c0 + lane + 1] - o0;
                 }
                 longest = max(longest, __reduce_max_sync(0xffffffffu, len0));
+MSPAI_LOOP
                 for (int q = 0; q < cn; q += 8) {
                     int64_t b[2];
                     int o[2], len[2], row[2] = {0, 0};
@@ -806,6 +823,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                     }
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
+MSPAI_LOOP
                         for (int t = l8; t < len[h]; t += 8) {
                             const int e = o[h] + t;
                             if (t != l8) {
@@ -821,11 +839,13 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                 }
             }
         }
+MSPAI_LOOP
         for (int jj = g.warp(); G::kWarps > 1 && jj < n; jj += G::kWarps) {
             const int j = scol(jj);
             const int64_t base = pb.cptr[j];
             const int o = s.off[jj];
             const int len = s.off[jj + 1] - o;
+MSPAI_LOOP
             for (int t = lane; t < len; t += 32) {
                 const int e = o + t;
                 const int row = pb.cidx[base + t];
@@ -838,10 +858,12 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
             uint64_t* ka = kdst;
             uint64_t* kb = ka + E;
             int* offs = reinterpret_cast<int*>(kb + E);
+MSPAI_LOOP
             for (int i = g.rank(); i <= n; i += G::kSize)
                 offs[i] = s.off[i];
             g.sync();
             const uint64_t* sorted = group_merge_runs(g, ka, kb, E, offs, n);
+MSPAI_LOOP
             for (int i = g.rank(); i < E; i += G::kSize)
                 s.keys[i] = sorted[i];
             g.sync();
@@ -850,16 +872,19 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
             // bitonic sort of the keys padded to a power of two: in the
             // shared area when it fits, else in place in the global slot
             const int L = next_pow2(E > 0 ? E : 1);
+MSPAI_LOOP
             for (int i = E + g.rank(); i < L; i += G::kSize)
                 s.keys[i] = ~uint64_t(0);
             g.sync();
             if (s.Wfast && static_cast<size_t>(L) * sizeof(uint64_t) <=
                                static_cast<size_t>(s.wfast_elems) * sizeof(T)) {
                 uint64_t* ks = reinterpret_cast<uint64_t*>(s.Wfast);
+MSPAI_LOOP
                 for (int i = g.rank(); i < L; i += G::kSize)
                     ks[i] = s.keys[i];
                 g.sync();
                 group_bitonic_sort(g, ks, L);
+MSPAI_LOOP
                 for (int i = g.rank(); i < E; i += G::kSize)
                     s.keys[i] = ks[i];
                 g.sync();
@@ -871,10 +896,12 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
 
         PHASE_MARK(0);
         // ---- unique rows I, positions of entries, row runs
+MSPAI_LOOP
         for (int i = g.rank(); i < E; i += G::kSize)
             s.tmp[i] = (i == 0 || (s.keys[i] >> kEntryBits) != (s.keys[i - 1] >> kEntryBits)) ? 1 : 0;
         g.sync();
         const int m = group_exclusive_scan(g, s.tmp, E);
+MSPAI_LOOP
         for (int i = g.rank(); i < E; i += G::kSize) {
             const bool first = (i == 0 || (s.keys[i] >> kEntryBits) != (s.keys[i - 1] >> kEntryBits));
             const int u = first ? s.tmp[i] : s.tmp[i] - 1;
@@ -888,6 +915,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
             s.rstart[m] = E;
         g.sync();
         // row classes: shared rows (>= 2 entries) get dense row numbers
+MSPAI_LOOP
         for (int u = g.rank(); u < m; u += G::kSize)
             s.tmp[u] = (s.rstart[u + 1] - s.rstart[u]) >= 2 ? 1 : 0;
         g.sync();
@@ -920,6 +948,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
         // area holds the right-hand side of every singleton entry
         const bool fixed = (pb.ns == 0);
         if (fixed) {
+MSPAI_LOOP
             for (int e = g.rank(); e < E; e += G::kSize) {
                 const int u = s.pos[e];
                 const bool shared = (s.rstart[u + 1] - s.rstart[u]) >= 2;
@@ -929,29 +958,34 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                             target_value(pb, bs * col + c, s.I[u]);
                 s.pos[e] = shared ? s.tmp[u] : -1;
             }
+MSPAI_LOOP
             for (int u = g.rank(); u < m; u += G::kSize)
                 if (s.rstart[u + 1] - s.rstart[u] >= 2)
                     s.srow[s.tmp[u]] = u;
         }
         if (!qru) {
             if (structured) {
+MSPAI_LOOP
                 for (int i = g.rank(); i < S * wcols; i += G::kSize) {
                     const int c = i / S, r = i - c * S;
                     W[r0 + r + static_cast<size_t>(c) * ld] = T(0);
                 }
             }
             else {
+MSPAI_LOOP
                 for (int i = g.rank(); i < mw * wcols; i += G::kSize)
                     W[i] = T(0);
             }
             g.sync();
             // shared entries
             if (fixed) {
+MSPAI_LOOP
                 for (int e = g.rank(); e < E; e += G::kSize) {
                     const int cd = s.pos[e];
                     if (cd >= 0)
                         W[static_cast<size_t>(s.ejj[e]) * ld + r0 + cd] = static_cast<T>(s.ev[e]);
                 }
+MSPAI_LOOP
                 for (int t = g.rank(); t < S * nrhs; t += G::kSize) {
                     const int c = t / S, d = t - c * S;
                     rhs[r0 + d + static_cast<size_t>(c) * ld] =
@@ -959,6 +993,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                 }
             }
             else {
+MSPAI_LOOP
                 for (int i = g.rank(); i < E; i += G::kSize) {
                     const int e = static_cast<int>(s.keys[i] & kEntryMask);
                     const int u = s.pos[e];
@@ -978,6 +1013,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
             bool folded = false;
             if constexpr (G::kWarps == 1) {
                 folded = nrhs == 1 && longest <= 8 && !structured;
+#pragma unroll 1
                 for (int j0 = 0; folded && j0 < n; j0 += 4) {
                     const int jj = j0 + (lane >> 3);
                     const int e = jj < n ? s.off[jj] + (lane & 7) : 0;
@@ -1005,9 +1041,11 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                     }
                 }
             }
+MSPAI_LOOP
             for (int jj = g.warp(); !folded && jj < n; jj += G::kWarps) {
                 double sig = 0.0;
                 double tb[kMaxBlockSize] = {};
+MSPAI_LOOP
                 for (int e = s.off[jj] + lane; e < s.off[jj + 1]; e += 32) {
                     int u = 0;
                     const bool single =
@@ -1071,6 +1109,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                 T* rp = s.Wfast;
                 T* rh = s.Wfast + static_cast<size_t>(n) * (n + 1) / 2;
                 group_pack_r<T>(g, Rg, n, n, rp);
+MSPAI_LOOP
                 for (int t = g.rank(); t < n * nrhs; t += G::kSize)
                     rh[t] = rhs_s[t];
                 g.sync();
@@ -1092,6 +1131,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                 T* rp = s.Wfast;
                 T* rh = s.Wfast + static_cast<size_t>(n) * (n + 1) / 2;
                 group_pack_r<T>(g, W, ld, n, rp);
+MSPAI_LOOP
                 for (int t = g.rank(); t < n * nrhs; t += G::kSize) {
                     const int c = t / n, i = t - c * n;
                     rh[t] = rhs[i + static_cast<size_t>(c) * ld];
@@ -1170,6 +1210,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                         group_normal_correction_rl<T>(g, rq, n, s.rinv,
                                                       s.gv + static_cast<size_t>(c) * n);
                     double d2 = 0.0, x2 = 0.0;
+MSPAI_LOOP
                     for (int t = g.rank(); t < n * nrhs; t += G::kSize) {
                         const double x1 = s.x[t] + s.gv[t];
                         d2 += s.gv[t] * s.gv[t];
@@ -1193,10 +1234,12 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
             double d2_prev = 0.0;
             for (int it = 0; it < pb.refine; it++) {
                 g.sync();
+MSPAI_LOOP
                 for (int t = g.warp(); t < n * nrhs; t += G::kWarps) {
                     const int c = t / n, jj = t - c * n;
                     const double* rc = s.r + static_cast<size_t>(c) * m;
                     double d = 0.0;
+MSPAI_LOOP
                     for (int e = s.off[jj] + lane; e < s.off[jj + 1]; e += 32)
                         d += s.ev[e] * rc[s.pos[e]];
                     d = warp_sum(d);
@@ -1206,10 +1249,12 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                 g.sync();
                 if (qru) {
                     // R is in W's column order: permute, correct, permute back
+MSPAI_LOOP
                     for (int t = g.rank(); t < n; t += G::kSize)
                         s.qperm[t] = s.gv[s.qpos[t]];
                     g.sync();
                     group_normal_correction<T>(g, W, ld, n, s.qperm);
+MSPAI_LOOP
                     for (int t = g.rank(); t < n; t += G::kSize)
                         s.gv[s.qpos[t]] = s.qperm[t];
                     g.sync();
@@ -1225,6 +1270,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                     }
                 }
                 double d2 = 0.0, x2 = 0.0;
+MSPAI_LOOP
                 for (int t = g.rank(); t < n * nrhs; t += G::kSize) {
                     const double x1 = s.x[t] + s.gv[t];
                     d2 += s.gv[t] * s.gv[t];
@@ -1268,12 +1314,14 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
         }
         else {
             // block rows of I (rows < n) are non-decreasing in u
+MSPAI_LOOP
             for (int u = g.rank(); u < m; u += G::kSize) {
                 const int r = s.I[u];
                 s.tmp[u] = (r < pb.n && (u == 0 || r / bs != s.I[u - 1] / bs)) ? 1 : 0;
             }
             g.sync();
             const int nb_i = group_exclusive_scan(g, s.tmp, m);
+MSPAI_LOOP
             for (int u = g.rank(); u < m; u += G::kSize) {
                 const int r = s.I[u];
                 if (r < pb.n && (u == 0 || r / bs != s.I[u - 1] / bs))
@@ -1305,6 +1353,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
         if constexpr (G::kWarps == 1) {
             hashed = s.ctab != nullptr;
             if (hashed) {
+MSPAI_LOOP
                 for (int i = lane; i < kCandTable; i += 32)
                     s.ctab[i] = -1;
                 __syncwarp();
@@ -1312,6 +1361,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
             const int grp = lane >> 3, l8 = lane & 7;
             auto insert = [&](int c) {
                 uint32_t h = (static_cast<uint32_t>(c) * 2654435761u) >> (32 - kCandTableBits);
+#pragma unroll 1
                 for (int probe = 0; probe < kCandTable; probe++) {
                     const int old = atomicCAS(&s.ctab[h], -1, c);
                     if (old == c)
@@ -1326,6 +1376,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                 }
                 atomicAdd(&g.sc->i[1], cap.cmax + 1);  // the table is full
             };
+MSPAI_LOOP
             for (int u0 = 0; hashed && u0 < nl; u0 += 32) {
                 const int un = min(32, nl - u0);
                 int64_t b0 = 0;
@@ -1337,6 +1388,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                         len0 = static_cast<int>(__ldg(pb.rptr + l + 1) - b0);
                     }
                 }
+MSPAI_LOOP
                 for (int q = 0; q < un; q += 8) {
                     int64_t b[2];
                     int len[2], c[2] = {0, 0};
@@ -1350,11 +1402,13 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
                     }
 #pragma unroll
                     for (int h = 0; h < 2; h++)
+MSPAI_LOOP
                         for (int t = l8; t < len[h]; t += 8)
                             insert(t == l8 ? c[h] : __ldg(pb.rcol + b[h] + t));
                 }
             }
         }
+MSPAI_LOOP
         for (int u = g.warp(); !hashed && u < nl; u += G::kWarps) {
             int r0, r1;
             if (bs == 1) {
@@ -1370,6 +1424,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
             for (int r = r0; r < r1; r++) {
                 const int64_t b0 = pb.rptr[r];
                 const int len = static_cast<int>(pb.rptr[r + 1] - b0);
+MSPAI_LOOP
                 for (int t = lane; t < len; t += 32) {
                     const int c = pb.rcol[b0 + t] / bs;
                     const uint32_t bit = 1u << (c & 31);
@@ -1386,6 +1441,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
         const int nu = g.sc->i[1];
         const int T_c = min(nu, cap.cmax);
         // clear the bit vector for the next use (every set bit is listed)
+MSPAI_LOOP
         for (int t = g.rank(); !hashed && t < T_c; t += G::kSize)
             s.bmap[s.cand[t] >> 5] = 0u;
         g.sync();
@@ -1394,11 +1450,13 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
             break;
         }
         const int LC = next_pow2(T_c > 0 ? T_c : 1);
+MSPAI_LOOP
         for (int i = T_c + g.rank(); i < LC; i += G::kSize)
             s.cand[i] = 0x7fffffff;
         g.sync();
         group_bitonic_sort(g, s.cand, LC);
         // keep candidates not in J (and, scalar only, in UP(:,col))
+MSPAI_LOOP
         for (int i = g.rank(); i < T_c; i += G::kSize) {
             const int c = s.cand[i];
             int keep = 1;
@@ -1422,38 +1480,49 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
         g.sync();
         // compact (ascending) into rho[] used as int storage, then back to cand
         int32_t* jt = reinterpret_cast<int32_t*>(s.rho);
+MSPAI_LOOP
         for (int i = g.rank(); i < T_c; i += G::kSize)
             if (s.ctmp[i + 1] > s.ctmp[i])
                 jt[s.ctmp[i]] = s.cand[i];
         g.sync();
         if (nt == 0)
             break;  // no candidates: Augment_Sparsity returns false
+MSPAI_LOOP
         for (int t = g.rank(); t < nt; t += G::kSize)
             s.cand[t] = jt[t];
         g.sync();
         // rho per candidate (one thread per candidate)
         const double res2 = res * res;
+MSPAI_LOOP
         for (int t = g.rank(); t < nt; t += G::kSize) {
             const int j = s.cand[t];
             if (bs == 1) {
                 double a2 = 0.0, num = 0.0;
                 const int64_t pe = pb.cptr[j + 1];
-                for (int64_t p = pb.cptr[j]; p < pe; p += 4) {  // four entries in flight
-                    int row[4];
-                    double v[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        row[q] = p + q < pe ? __ldg(pb.cidx + p + q) : -1;
-                        v[q] = p + q < pe ? __ldg(pb.cval + p + q) : 0.0;
+                if constexpr (G::kWarps == 1) {
+                    int64_t p = pb.cptr[j];
+                    int row = p < pe ? __ldg(pb.cidx + p) : 0;
+                    double v = p < pe ? __ldg(pb.cval + p) : 0.0;
+#pragma unroll 1
+                    while (p < pe) {
+                        p++;  // the next entry is on its way
+                        const int row1 = p < pe ? __ldg(pb.cidx + p) : 0;
+                        const double v1 = p < pe ? __ldg(pb.cval + p) : 0.0;
+                        a2 += v * v;
+                        const int u = lower_bound_i32(s.I, m, row);
+                        if (u < m && s.I[u] == row)
+                            num += s.r[u] * v;
+                        row = row1;
+                        v = v1;
                     }
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        if (row[q] < 0)
-                            break;
-                        a2 += v[q] * v[q];
-                        const int u = lower_bound_i32(s.I, m, row[q]);
-                        if (u < m && s.I[u] == row[q])
-                            num += s.r[u] * v[q];
+                }
+                else {
+                    for (int64_t p = pb.cptr[j]; p < pe; p++) {
+                        const double v = pb.cval[p];
+                        a2 += v * v;
+                        const int u = lower_bound_i32(s.I, m, pb.cidx[p]);
+                        if (u < m && s.I[u] == pb.cidx[p])
+                            num += s.r[u] * v;
                     }
                 }
                 const double ajn = sqrt(a2);
@@ -1496,6 +1565,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
         {
             // algorithmic work of the candidate scan: 4 flops per entry
             int ce = 0;
+MSPAI_LOOP
             for (int t = g.rank(); t < nt; t += G::kSize)
                 for (int a = 0; a < bs; a++)
                     ce += static_cast<int>(pb.cptr[s.cand[t] * bs + a + 1] -
@@ -1523,6 +1593,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
             for (int sel = 0; sel < pb.mn && sel < nt; sel++) {
                 double best = 0.0;
                 int bj = 0x7fffffff, bt = -1;
+MSPAI_LOOP
                 for (int t = lane; t < nt; t += 32) {
                     const double rv = s.rho[t];
                     const int j = s.cand[t];
@@ -1601,6 +1672,7 @@ __device__ void solve_column(const G& g, const Problem& pb, const Caps& cap, Slo
         }
         int nonfinite = 0;
         const double* xc = s.x + static_cast<size_t>(c) * n;
+MSPAI_LOOP
         for (int t = g.rank(); t < n; t += G::kSize) {
             const double v = xc[t];
             if (!isfinite(v))
