@@ -566,6 +566,8 @@ __device__ bool gather_shared(CgShared& sh, const Problem& pb, int col, char* ba
                 d0[jj] += v * v;
             __syncwarp();
         }
+        // the next pass reads the counts that other lanes have written in this one
+        __syncwarp();
     }
     __syncthreads();
     g.n = n;
