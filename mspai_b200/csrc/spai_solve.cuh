@@ -1348,7 +1348,10 @@ MSPAI_LOOP
         // slots in shared memory: a hash set of kCandTable columns instead of the
         // bit vector (its atomics went to the L2), eight lanes a row, eight rows'
         // first entries in flight.  More columns than the list holds: status 3
-        // below, and the caller gives the column to a larger slot.
+        // below, and the caller gives the column to a larger slot.  The scan ends
+        // as soon as that is certain (a row of more entries says so by itself), so
+        // at most the list's length and one column a lane are inserted and a probe
+        // always meets a free place.
         bool hashed = false;
         if constexpr (G::kWarps == 1) {
             hashed = s.ctab != nullptr;
@@ -1359,6 +1362,7 @@ MSPAI_LOOP
                 __syncwarp();
             }
             const int grp = lane >> 3, l8 = lane & 7;
+            const volatile int* found = &g.sc->i[1];
             auto insert = [&](int c) {
                 uint32_t h = (static_cast<uint32_t>(c) * 2654435761u) >> (32 - kCandTableBits);
 #pragma unroll 1
@@ -1374,10 +1378,10 @@ MSPAI_LOOP
                     }
                     h = (h + 1) & (kCandTable - 1);
                 }
-                atomicAdd(&g.sc->i[1], cap.cmax + 1);  // the table is full
             };
+            bool lost = false;  // more candidates than the list holds (warp-uniform)
 MSPAI_LOOP
-            for (int u0 = 0; hashed && u0 < nl; u0 += 32) {
+            for (int u0 = 0; hashed && !lost && u0 < nl; u0 += 32) {
                 const int un = min(32, nl - u0);
                 int64_t b0 = 0;
                 int len0 = 0;
@@ -1388,8 +1392,9 @@ MSPAI_LOOP
                         len0 = static_cast<int>(__ldg(pb.rptr + l + 1) - b0);
                     }
                 }
+                lost = __any_sync(0xffffffffu, len0 > cap.cmax);
 MSPAI_LOOP
-                for (int q = 0; q < un; q += 8) {
+                for (int q = 0; !lost && q < un; q += 8) {
                     int64_t b[2];
                     int len[2], c[2] = {0, 0};
 #pragma unroll
@@ -1403,10 +1408,13 @@ MSPAI_LOOP
 #pragma unroll
                     for (int h = 0; h < 2; h++)
 MSPAI_LOOP
-                        for (int t = l8; t < len[h]; t += 8)
+                        for (int t = l8; t < len[h] && *found <= cap.cmax; t += 8)
                             insert(t == l8 ? c[h] : __ldg(pb.rcol + b[h] + t));
+                    lost = __any_sync(0xffffffffu, *found > cap.cmax);
                 }
             }
+            if (lost && lane == 0)
+                g.sc->i[1] = cap.cmax + 1;
         }
 MSPAI_LOOP
         for (int u = g.warp(); !hashed && u < nl; u += G::kWarps) {

@@ -82,6 +82,7 @@ constexpr int kShareN = 16;
 constexpr int kShareE = 112;      // 16 columns of a 7-point stencil
 constexpr int kShareMw = 44;      // rows of the folded matrix
 constexpr int kShareCand = 192;   // unique candidates
+static_assert(kShareCand + 32 < kCandTable, "a probe meets a free place: the scan ends here");
 
 struct ShareSlot {
     uint64_t keys[kShareE];
