@@ -238,6 +238,31 @@ int mspai_column_info(mspai_handle* h, double* resnorm, int32_t* steps, int32_t*
 /* Statistics of the last setup. */
 int mspai_get_stats(mspai_handle* h, mspai_stats* s);
 
+/* The column solvers of a setup, in the order of mspai_solver_columns. */
+typedef enum {
+    MSPAI_SOLVER_SMALL_QR = 0,     /* eight lanes per column, Householder QR         */
+    MSPAI_SOLVER_WARP = 1,         /* a warp per column, Householder QR              */
+    MSPAI_SOLVER_ADAPTIVE = 2,     /* a warp per adaptive column, shared memory      */
+    MSPAI_SOLVER_SPARSE_SMALL = 3, /* sparse normal equations, elimination           */
+    MSPAI_SOLVER_SPARSE_25K = 4,   /* ... Chebyshev iteration, slots of 25 KB,       */
+    MSPAI_SOLVER_SPARSE_42K = 5,   /* 42 KB                                          */
+    MSPAI_SOLVER_SPARSE_104K = 6,  /* and 104 KB                                     */
+    MSPAI_SOLVER_FIXED = 7,        /* dense factorizations of fixed patterns ...     */
+    MSPAI_SOLVER_FIXED_LARGE = 8,  /* ... with the largest arena                     */
+    MSPAI_SOLVER_GENERAL = 9,      /* a CTA per column, Householder QR               */
+    MSPAI_SOLVER_BLOCK_SMALL = 10, /* block columns, eight lanes each,               */
+    MSPAI_SOLVER_BLOCK_64 = 11,    /* 64 threads each                                */
+    MSPAI_SOLVER_BLOCK_256 = 12,   /* and 256 threads each                           */
+    MSPAI_SOLVERS = 13
+} mspai_solver;
+
+/*
+ * Problem columns that the last setup handed to each solver (counts[MSPAI_SOLVERS]).
+ * A solver hands on what it does not take, so a column counts once for every
+ * solver that it came to.
+ */
+int mspai_solver_columns(mspai_handle* h, int64_t* counts);
+
 /*
  * Adjoint of the last setup for the loss
  *     L = ||C M - B||_F^2 + sum_k gbar_k^T m_k        (gbar optional)

@@ -75,7 +75,13 @@ EXPORTED = [
     "mspai_probing_assemble", "mspai_pattern_generate", "mspai_row_structure",
     "mspai_measure_fma_peak", "mspai_setup_fixed_noalloc", "mspai_block_pattern_generate",
     "mspai_pattern_power2", "mspai_get_tuning", "mspai_set_tuning", "mspai_pattern_powers",
+    "mspai_solver_columns",
 ]
+
+# the solvers of mspai_solver_columns, in order
+SOLVERS = ("small_qr", "warp", "adaptive", "sparse_small", "sparse_25k", "sparse_42k",
+           "sparse_104k", "fixed", "fixed_large", "general", "block_small", "block_64",
+           "block_256")
 
 _lib = None
 
@@ -117,6 +123,8 @@ def load() -> ctypes.CDLL:
     lib.mspai_column_info.restype = I
     lib.mspai_get_stats.argtypes = [V, P(mspai_stats)]
     lib.mspai_get_stats.restype = I
+    lib.mspai_solver_columns.argtypes = [V, P(ctypes.c_int64)]
+    lib.mspai_solver_columns.restype = I
     lib.mspai_adjoint.argtypes = [V, P(mspai_csc), P(mspai_csc), V, V, V,
                                   P(ctypes.c_double), ctypes.c_int32]
     lib.mspai_adjoint.restype = I

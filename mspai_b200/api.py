@@ -286,6 +286,13 @@ class Handle:
             "factor_reuse_columns": s.factor_reuse_columns,
         }
 
+    def solver_columns(self) -> dict:
+        """Problem columns that the last setup handed to each column solver
+        (mspai_solver_columns)."""
+        c = (ctypes.c_int64 * len(_lib.SOLVERS))()
+        self._check(self._lib.mspai_solver_columns(self._h, c))
+        return dict(zip(_lib.SOLVERS, c))
+
     def adjoint(self, C: MatrixLike, B: Optional[MatrixLike] = None,
                 gbar: Optional[np.ndarray] = None, residual_weight: float = 1.0):
         """Gradient of w ||C M - B||_F^2 + gbar . M (w = residual_weight) with

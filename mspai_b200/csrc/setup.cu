@@ -143,6 +143,10 @@ struct mspai_handle {
     int64_t list_len[kLists] = {};   // columns listed per work list in the last setup
     int64_t tiny_len = 0;            // ... in the sparse solvers' list of small columns
     int64_t small_len = 0;           // ... and in the small QR's
+    // columns handed to each solver in the last setup: a number, plus the device
+    // counter handed_at (-1: none), which stays until the next setup
+    int64_t handed[MSPAI_SOLVERS] = {};
+    int handed_at[MSPAI_SOLVERS] = {};
 };
 
 static int set_err(mspai_handle* h, int code, const char* fmt, ...)
@@ -721,6 +725,10 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
     for (int k = 0; k < kLists; k++)
         h->list_len[k] = 0;
     bool timed[kKernels] = {false, false, false, false};
+    for (int k = 0; k < MSPAI_SOLVERS; k++) {
+        h->handed[k] = 0;
+        h->handed_at[k] = -1;
+    }
     h->used_fixed = use_fixed;
     // general CTA solver over `count` listed columns with the given caps
     auto run_cta = [&](int b, const Caps& cap, int32_t* list, int count, int32_t* counter,
@@ -735,6 +743,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             CUDA_TRY(h, cudaMemsetAsync(h->scratch.p, 0, need, st));
         CUDA_TRY(h, cudaMemsetAsync(counter, 0, sizeof(int32_t), st));
         h->launches++;
+        h->handed[MSPAI_SOLVER_GENERAL] += count;
         CUDA_TRY(h, mspai::launch_cta_solve(elem_b, wsm, prm->batched != 0, pbb, cap, out, list,
                                             count, counter, h->scratch.as<char>(),
                                             h->scratch.bytes, st, &grid));
@@ -758,6 +767,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
         h->stats.bucket_columns[0] = nsmall;
     }
     h->small_len = nsmall;
+    h->handed[MSPAI_SOLVER_SMALL_QR] = nsmall;
     const int tiny = rule.tiny_list > 0 ? hc[3] : 0;  // small columns of the sparse solvers
     h->tiny_len = tiny;
     if (tiny > 0) {  // their sizes belong to the fixed-pattern bucket
@@ -800,6 +810,9 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             CUDA_TRY(h, cudaMemsetAsync(bc, 0, 5 * sizeof(int32_t), st));
             CUDA_TRY(h, cudaEventRecord(h->evb[2 * b], st));
             h->launches += 3;
+            h->handed[MSPAI_SOLVER_BLOCK_SMALL] = count;
+            h->handed_at[MSPAI_SOLVER_BLOCK_64] = static_cast<int>(bc - dcnt);
+            h->handed_at[MSPAI_SOLVER_BLOCK_256] = static_cast<int>(bc + 1 - dcnt);
             CUDA_TRY(h, mspai::launch_block_solve(elem, pb, out, list, count, rest, bc, st));
             CUDA_TRY(h, cudaEventRecord(h->evb[2 * b + 1], st));
             timed[b] = true;
@@ -840,6 +853,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
                 int32_t* rest = h->lists.as<int32_t>() + static_cast<size_t>(kLists) * nprob;
                 CUDA_TRY(h, cudaMemsetAsync(dcnt + 28, 0, sizeof(int32_t), st));
                 h->launches++;
+                h->handed[MSPAI_SOLVER_ADAPTIVE] = count;
                 CUDA_TRY(h, mspai::launch_warp_adaptive(pbb, out, list, count, counter, rest,
                                                         dcnt + 28, st));
                 CUDA_TRY(h, cudaMemcpyAsync(&left, dcnt + 28, sizeof(int32_t),
@@ -854,6 +868,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
                 if (adaptive)  // the candidate bit vectors of the slots start cleared
                     CUDA_TRY(h, cudaMemsetAsync(h->scratch.p, 0, need, st));
                 h->launches++;
+                h->handed[MSPAI_SOLVER_WARP] = left;
                 CUDA_TRY(h, mspai::launch_warp_solve_global(elem_b, pbb, cap, out, list, left,
                                                             counter, h->scratch.as<char>(),
                                                             h->scratch.bytes, st, &grid));
@@ -866,6 +881,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             if (nsmall == 0)
                 CUDA_TRY(h, cudaEventRecord(h->evb[0], st));
             h->launches++;
+            h->handed[MSPAI_SOLVER_WARP] = count;
             CUDA_TRY(h, mspai::launch_warp_solve(elem_b, pbb, cap, out, list, count, counter, st,
                                                  &grid));
             CUDA_TRY(h, cudaEventRecord(h->evb[1], st));
@@ -899,6 +915,10 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
                         break;
                     rest = h->lists.as<int32_t>() + static_cast<size_t>(kLists + k % 2) * nprob;
                     h->launches++;
+                    if (fcount)
+                        h->handed_at[MSPAI_SOLVER_SPARSE_25K + k] = static_cast<int>(fcount - dcnt);
+                    else
+                        h->handed[MSPAI_SOLVER_SPARSE_25K + k] = hc[1];
                     CUDA_TRY(h, mspai::launch_sparse_solve(elem, c.kind, c.slot_bytes, pb, out,
                                                            flist, fcount, hc[1], sc + 4 + k, rest,
                                                            sc + k, st));
@@ -912,6 +932,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
                         h->lists.as<int32_t>() + static_cast<size_t>(rule.tiny_list) * nprob;
                     int32_t* rc3 = sc + std::max(k - 1, 0);
                     h->launches++;
+                    h->handed[MSPAI_SOLVER_SPARSE_SMALL] = tiny;
                     CUDA_TRY(h, mspai::launch_sparse_solve(8, mspai::SparseLaunch::kTiny,
                                                            kSparseTinySlot, pb, out, tl, nullptr,
                                                            tiny, sc + 7, rest, rc3, st));
@@ -920,6 +941,10 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
                 }
             }
             h->launches++;
+            if (fcount)
+                h->handed_at[MSPAI_SOLVER_FIXED] = static_cast<int>(fcount - dcnt);
+            else
+                h->handed[MSPAI_SOLVER_FIXED] = count;
             CUDA_TRY(h, mspai::launch_fixed_solve(elem, h->fixed_arena, pb, out, flist, fcount,
                                                   count, counter, ovf_a, cnt, h->rglob.p, relems,
                                                   grid_max, st, &grid));
@@ -934,6 +959,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             int32_t ho[2] = {0, 0};
             CUDA_TRY(h, cudaMemcpyAsync(ho, cnt, sizeof(ho), cudaMemcpyDeviceToHost, st));
             CUDA_TRY(h, cudaStreamSynchronize(st));
+            h->handed[MSPAI_SOLVER_FIXED_LARGE] = ho[0];
             h->list_len[2] = ho[0];
             h->list_len[3] = ho[1];
             h->stats.bucket_columns[1] = count - ho[0];
@@ -1212,6 +1238,21 @@ int mspai_column_info(mspai_handle* h, double* resnorm, int32_t* steps, int32_t*
         CUDA_TRY(h, cudaMemcpyAsync(status, h->status.p, sizeof(int32_t) * h->n,
                                     cudaMemcpyDeviceToHost, st));
     CUDA_TRY(h, cudaStreamSynchronize(st));
+    return MSPAI_OK;
+}
+
+int mspai_solver_columns(mspai_handle* h, int64_t* counts)
+{
+    if (!h || !h->have_result)
+        return h ? set_err(h, MSPAI_ERR_STATE, "no setup result") : MSPAI_ERR_STATE;
+    if (!counts)
+        return set_err(h, MSPAI_ERR_PARAM, "counts is required");
+    CUDA_TRY(h, cudaSetDevice(h->device));
+    int32_t c[64];
+    CUDA_TRY(h, cudaMemcpyAsync(c, h->counters.p, sizeof(c), cudaMemcpyDeviceToHost, h->stream));
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    for (int k = 0; k < MSPAI_SOLVERS; k++)
+        counts[k] = h->handed[k] + (h->handed_at[k] >= 0 ? c[h->handed_at[k]] : 0);
     return MSPAI_OK;
 }
 
