@@ -11,7 +11,8 @@
 // are FP32, FP64 steps otherwise.  A row with one entry v of column j has
 // r = -v x_j and C lambda = v lambda_j, so its gradient needs no row at all:
 //     dL/dv = 2 w v x_j^2 - 2 v x_j lambda_j.
-// Columns that do not fit or are not certified go to the general adjoint.
+// A column that does not fit the slot goes to the next launch (a larger one), one
+// that is not certified to the general adjoint at once.
 //   Bound: the passes over the entries of C and the FP64 atomics on dC.  12,000
 //   ragged columns of 134 unknowns and 2,500 entries with a gbar: 17.9 ms in the
 //   general adjoint, 2.4 ms here.
@@ -24,14 +25,15 @@ namespace mspai {
 namespace {
 
 template <class T, int NW, int K>
-__device__ bool adjoint_column(CgShared& sh, const Problem& pb, const AdjointIO& io, int col,
-                               char* base, int cap)
+__device__ Taken adjoint_column(CgShared& sh, const Problem& pb, const AdjointIO& io, int col,
+                                char* base, int cap, int widest)
 {
     constexpr int NT = 32 * NW, LG = NT / 8;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, grp = lane >> 3, l8 = lane & 7;
     SharedEntries g;
-    if (!gather_shared<NW>(sh, pb, col, base, cap, LG + NT * (K - 1), g))
-        return false;
+    const Taken fit = gather_shared<NW>(sh, pb, col, base, cap, LG + NT * (K - 1), widest, g);
+    if (fit != Taken::kYes)
+        return fit;
     const int n = g.n;
     // ---- the rest of the slot: M's values by position, the residual of the
     // shared rows, gbar by position, one bit per entry of C(:, J) (shared)
@@ -41,11 +43,11 @@ __device__ bool adjoint_column(CgShared& sh, const Problem& pb, const AdjointIO&
     uint32_t* bits = reinterpret_cast<uint32_t*>(gb + (io.gbar ? n : 0));
     const int words = (g.E + 31) / 32;
     if (reinterpret_cast<char*>(bits + words) > base + g.free_hi)
-        return false;
+        return Taken::kLarger;
     int at[K], parity = 0;
     const int nlong = column_slots<NW, K>(sh, n, at);
     if (!column_scales<NW, K>(g, at))
-        return false;
+        return Taken::kNo;
     // ---- r = b - C m on the shared rows; ||r||^2, the target outside of I
     double part = 0.0, gx = 0.0;
 #pragma unroll
@@ -84,7 +86,7 @@ __device__ bool adjoint_column(CgShared& sh, const Problem& pb, const AdjointIO&
     if (io.gbar) {
         __syncthreads();
         if (cg_solve<T, NW, K>(sh, parity, g, at, nlong, gb, nullptr) < 0)
-            return false;
+            return Taken::kNo;
     }
     else {
         __syncthreads();
@@ -156,15 +158,15 @@ __device__ bool adjoint_column(CgShared& sh, const Problem& pb, const AdjointIO&
     cta_sum2<NW>(sh, parity, part, gx);
     if (tid == 0)
         io.loss[col] = io.wres * part + gx;
-    return true;
+    return Taken::kYes;
 }
 
 template <class T, int NW, int K, int MINB>
 __global__ void __launch_bounds__(32 * NW, MINB)
     adjoint_sparse_kernel(Problem pb, AdjointIO io, const int32_t* __restrict__ list,
                           const int32_t* __restrict__ count_dev, int count_host,
-                          int32_t* __restrict__ counter, int32_t* __restrict__ ovf_list,
-                          int32_t* __restrict__ ovf_count, int slot_bytes)
+                          int32_t* __restrict__ counter, WorkList larger, WorkList refused,
+                          int slot_bytes, int widest)
 {
     extern __shared__ __align__(16) char smem[];
     __shared__ CgShared sh;
@@ -178,15 +180,19 @@ __global__ void __launch_bounds__(32 * NW, MINB)
         if (t >= count)
             break;
         const int col = list[t];
-        if (!adjoint_column<T, NW, K>(sh, pb, io, col, smem, slot_bytes) && threadIdx.x == 0)
-            ovf_list[atomicAdd(ovf_count, 1)] = col;
+        const Taken taken = adjoint_column<T, NW, K>(sh, pb, io, col, smem, slot_bytes, widest);
+        if (taken != Taken::kYes && threadIdx.x == 0) {
+            const WorkList& to = taken == Taken::kLarger ? larger : refused;
+            to.list[atomicAdd(to.count, 1)] = col;
+        }
     }
 }
 
 template <class T, int NW, int K, int MINB>
-cudaError_t launch_t(int slot_bytes, const Problem& pb, const AdjointIO& io, const int32_t* list,
-                     const int32_t* count_dev, int count_host, int32_t* counter, int32_t* ovf_list,
-                     int32_t* ovf_count, cudaStream_t st)
+cudaError_t launch_t(int slot_bytes, int widest, const Problem& pb, const AdjointIO& io,
+                     const int32_t* list, const int32_t* count_dev, int count_host,
+                     int32_t* counter, const WorkList& larger, const WorkList& refused,
+                     cudaStream_t st)
 {
     auto kern = adjoint_sparse_kernel<T, NW, K, MINB>;
     cudaError_t e =
@@ -200,29 +206,29 @@ cudaError_t launch_t(int slot_bytes, const Problem& pb, const AdjointIO& io, con
     if (per_sm < 1)
         return cudaErrorInvalidConfiguration;
     const int grid = std::max(1, std::min(per_sm * num_sms(), count_host));
-    kern<<<grid, 32 * NW, slot_bytes, st>>>(pb, io, list, count_dev, count_host, counter, ovf_list,
-                                            ovf_count, slot_bytes);
+    kern<<<grid, 32 * NW, slot_bytes, st>>>(pb, io, list, count_dev, count_host, counter, larger,
+                                            refused, slot_bytes, widest);
     return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_adjoint_sparse(const Problem& pb, const AdjointIO& io, const int32_t* list,
-                                  int count, int32_t* const rest[2], int32_t* counts,
-                                  int32_t** left, int32_t** left_count, cudaStream_t st)
+                                  int count, int32_t* const rest[3], int32_t* counts,
+                                  cudaStream_t st)
 {
     // slots of six, four and two CTAs per SM
+    constexpr int kNarrow = 34 * 1024, kMiddle = 52 * 1024, kWide = 108 * 1024;
     const bool f = io.rstore && io.r_elem == 4;
     auto a = f ? launch_t<float, 4, 2, 6> : launch_t<double, 4, 2, 6>;
     auto b = f ? launch_t<float, 4, 3, 4> : launch_t<double, 4, 3, 4>;
     auto c = f ? launch_t<float, 4, 4, 2> : launch_t<double, 4, 4, 2>;
-    cudaError_t e = a(34 * 1024, pb, io, list, nullptr, count, counts + 3, rest[0], counts, st);
+    const WorkList refused{rest[0], counts}, r1{rest[1], counts + 1}, r2{rest[2], counts + 2};
+    cudaError_t e = a(kNarrow, kWide, pb, io, list, nullptr, count, counts + 3, r1, refused, st);
     if (e == cudaSuccess)
-        e = b(52 * 1024, pb, io, rest[0], counts, count, counts + 4, rest[1], counts + 1, st);
+        e = b(kMiddle, kWide, pb, io, r1.list, r1.count, count, counts + 4, r2, refused, st);
     if (e == cudaSuccess)
-        e = c(108 * 1024, pb, io, rest[1], counts + 1, count, counts + 5, rest[0], counts + 2, st);
-    *left = rest[0];
-    *left_count = counts + 2;
+        e = c(kWide, kWide, pb, io, r2.list, r2.count, count, counts + 5, refused, refused, st);
     return e;
 }
 

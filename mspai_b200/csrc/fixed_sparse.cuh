@@ -138,19 +138,30 @@ struct SharedEntries {
     double tg_val;
 };
 
-// Lays column `col` out in the slot; false (uniformly) when it has more than
-// nmax columns or does not fit.
+// What becomes of a column.
+enum class Taken {
+    kYes,
+    kLarger,  // it does not fit this slot
+    kNo       // it fits no slot, or the solver refuses it: the next slot would as well
+};
+
+constexpr int kWidestN = 400;  // columns of J in the largest slot
+
+// Lays column `col` out in the slot (uniformly); at most nmax columns of J.
+// widest: bytes of the largest slot that the launches use.
 template <int NW>
-__device__ bool gather_shared(CgShared& sh, const Problem& pb, int col, char* base, int cap,
-                              int nmax, SharedEntries& g)
+__device__ Taken gather_shared(CgShared& sh, const Problem& pb, int col, char* base, int cap,
+                               int nmax, int widest, SharedEntries& g)
 {
     constexpr int NT = 32 * NW;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     const int64_t p0 = pb.pptr[col];
     const int n = static_cast<int>(pb.pptr[col + 1] - p0);
-    if (n < 1 || n > nmax)
-        return false;
+    if (n < 1 || n > kWidestN)
+        return Taken::kNo;
+    if (n > nmax)
+        return Taken::kLarger;
     // ---- fixed part of the slot
     double* d0 = reinterpret_cast<double*>(base);
     double* gd = d0 + n;
@@ -163,8 +174,10 @@ __device__ bool gather_shared(CgShared& sh, const Problem& pb, int col, char* ba
     const int ra = static_cast<int>((reinterpret_cast<char*>(ccol + n) - base + 15) & ~15);
     const int64_t tg0 = pb.bptr ? pb.bptr[col] : 0;
     const int ntg = pb.bptr ? static_cast<int>(pb.bptr[col + 1] - tg0) : 1;
-    if (ra >= cap || ntg > kCgMaxTargets)
-        return false;
+    if (ntg > kCgMaxTargets)
+        return Taken::kNo;
+    if (ra >= cap)
+        return ra >= widest ? Taken::kNo : Taken::kLarger;
     if (tid == 0) {
         sh.entries = sh.longest = sh.distinct = sh.shared_entries = sh.over = 0;
     }
@@ -198,7 +211,7 @@ __device__ bool gather_shared(CgShared& sh, const Problem& pb, int col, char* ba
     __syncthreads();
     const int E = sh.entries;
     if (sh.longest > 0xffff || E < 1 || E > (1 << 20))
-        return false;
+        return Taken::kNo;
     // ---- the two bit maps: 8 to 16 bits per entry
     const int hb = max(10, 32 - __clz(8 * E - 1));
     const int mapw = 1 << (hb - 5);
@@ -206,7 +219,7 @@ __device__ bool gather_shared(CgShared& sh, const Problem& pb, int col, char* ba
     uint32_t* bm2 = bm1 + mapw;
     const int room = cap - ra - 8 * mapw;  // candidates, from the slot's end down
     if (room < 16 * n)
-        return false;
+        return widest - ra - 8 * mapw < 16 * n ? Taken::kNo : Taken::kLarger;
     // candidate c of warp w at cand[-(NW c + w)]
     uint2* cand = reinterpret_cast<uint2*>(base + cap) - 1 - warp;
 #pragma unroll 1
@@ -350,8 +363,6 @@ __device__ bool gather_shared(CgShared& sh, const Problem& pb, int col, char* ba
         ncmax = max(ncmax, sh.ncw[w]);
         nctot += sh.ncw[w];
     }
-    if (8 * NW * ncmax > room)
-        return false;
     // ---- candidates grouped by row: exact hash table (keys, counts by warp)
     const int ht = max(64, next_pow2(nctot + nctot / 2));
     const int htb = 31 - __clz(ht);
@@ -361,8 +372,10 @@ __device__ bool gather_shared(CgShared& sh, const Problem& pb, int col, char* ba
     uint32_t* cnt = key + ht;
     uint32_t* rcnt = reinterpret_cast<uint32_t*>(base + top);  // entries by warp of a row
     uint32_t* rfill = rcnt + smax;
-    if (8 * ht > top - ra)
-        return false;
+    // the candidates beside the bit maps, then beside the table and the rows' counts
+    const int need = ra + 8 * NW * ncmax + max(8 * mapw, 8 * ht + 8 * smax);
+    if (8 * NW * ncmax > room || 8 * ht > top - ra)
+        return need > widest ? Taken::kNo : Taken::kLarger;
 #pragma unroll 1
     for (int i = tid; i < ht / 4; i += NT) {
         reinterpret_cast<uint4*>(key)[i] = make_uint4(kNone, kNone, kNone, kNone);
@@ -426,7 +439,7 @@ __device__ bool gather_shared(CgShared& sh, const Problem& pb, int col, char* ba
     }
     __syncthreads();
     if (sh.over)
-        return false;
+        return Taken::kNo;
     if (warp == 0) {
         const uint32_t rows = cg_order(sh.bins, sh.rows, lane);
         if (lane == 0)
@@ -483,7 +496,7 @@ __device__ bool gather_shared(CgShared& sh, const Problem& pb, int col, char* ba
     }
     __syncthreads();
     if (sh.over)
-        return false;
+        return Taken::kNo;
     if (warp == 0) {
         cg_order(sh.bins, sh.cols, lane);
         __syncwarp();
@@ -514,7 +527,8 @@ __device__ bool gather_shared(CgShared& sh, const Problem& pb, int col, char* ba
     uint16_t* ec = reinterpret_cast<uint16_t*>(y + S);
     uint16_t* cr = ec + ns;
     if (20 * ns + 8 * S > top - ra || ns > 0xffff)
-        return false;
+        return 20 * ns + 8 * S > top - ra + widest - cap || ns > 0xffff ? Taken::kNo
+                                                                        : Taken::kLarger;
     __syncthreads();
 #pragma unroll 1
     for (int i = tid; i < n; i += NT)
@@ -595,7 +609,7 @@ __device__ bool gather_shared(CgShared& sh, const Problem& pb, int col, char* ba
     g.cand = cand;
     g.tg_rid = tg_rid;
     g.tg_val = tg_val;
-    return true;
+    return Taken::kYes;
 }
 
 }  // namespace mspai

@@ -30,7 +30,8 @@ constexpr int kBuckets = 3;    // size buckets of the planning kernel
 constexpr int kKernels = 4;    // solver launches per setup (timed separately)
 constexpr int kLists = 4;      // work lists: buckets + the overflow lists
 constexpr int kMoreLists = 5;  // ... two between the sparse solvers' launches, their small
-                               // columns, the small QR's columns and its tall ones
+                               // columns, the small QR's columns, its tall ones and, after
+                               // these, the sparse solvers' refused columns
 // Arena of the fixed-pattern solver's second launch (one CTA per SM): the
 // largest dynamic shared memory a CTA may have beside the solver's static part.
 constexpr int kFixedArenaLarge = 212 * 1024;
@@ -40,7 +41,8 @@ constexpr int kFixedArenaLarge = 212 * 1024;
 constexpr int kMixedFp64MaxN = 32;
 // Launches of the solvers on the sparse normal equations (fixed_cg.cu) over the
 // fixed-pattern bucket: shared memory of a column's CTA (25 KB: eight CTAs per
-// SM, 42 KB: five, 104 KB: two).  A column that does not fit goes on to the next.
+// SM, 42 KB: five, 104 KB: two).  A column that does not fit goes on to the next,
+// one that is refused to the dense factorizations.
 struct SparseClass {
     int slot_bytes;
     mspai::SparseLaunch kind;
@@ -906,39 +908,43 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             const int32_t* flist = list;
             const int32_t* fcount = nullptr;
             if (sparse) {
-                int32_t* sc = dcnt + 28;  // rest counts [4], then queue counters [4]
+                // columns for the second and the third slot, refused ones; queues
+                int32_t* sc = dcnt + 28;
                 CUDA_TRY(h, cudaMemsetAsync(sc, 0, 8 * sizeof(int32_t), st));
-                int32_t* rest = h->lists.as<int32_t>() + static_cast<size_t>(kLists) * nprob;
-                int k = 0;
+                int32_t* lists = h->lists.as<int32_t>();
+                auto more = [&](int k) { return lists + static_cast<size_t>(kLists + k) * nprob; };
+                const mspai::WorkList refused{more(4), sc + 2};
+                int widest = 0, classes = 0;
                 for (const SparseClass& c : kSparseClasses) {
-                    if (c.slot_bytes > h->fixed_arena || hc[1] == 0)
+                    if (c.slot_bytes > h->fixed_arena)
                         break;
-                    rest = h->lists.as<int32_t>() + static_cast<size_t>(kLists + k % 2) * nprob;
+                    widest = c.slot_bytes;
+                    classes++;
+                }
+                for (int k = 0; k < classes && hc[1] > 0; k++) {
+                    const SparseClass& c = kSparseClasses[k];
+                    const mspai::WorkList larger =
+                        k + 1 < classes ? mspai::WorkList{more(k), sc + k} : refused;
                     h->launches++;
                     if (fcount)
                         h->handed_at[MSPAI_SOLVER_SPARSE_25K + k] = static_cast<int>(fcount - dcnt);
                     else
                         h->handed[MSPAI_SOLVER_SPARSE_25K + k] = hc[1];
-                    CUDA_TRY(h, mspai::launch_sparse_solve(elem, c.kind, c.slot_bytes, pb, out,
-                                                           flist, fcount, hc[1], sc + 4 + k, rest,
-                                                           sc + k, st));
-                    flist = rest;
-                    fcount = sc + k;
-                    k++;
+                    CUDA_TRY(h, mspai::launch_sparse_solve(elem, c.kind, c.slot_bytes, widest, pb,
+                                                           out, flist, fcount, hc[1], sc + 4 + k,
+                                                           larger, refused, st));
+                    flist = larger.list;
+                    fcount = larger.count;
                 }
                 if (tiny > 0) {
-                    // what the small columns leave joins the rest
-                    const int32_t* tl =
-                        h->lists.as<int32_t>() + static_cast<size_t>(rule.tiny_list) * nprob;
-                    int32_t* rc3 = sc + std::max(k - 1, 0);
                     h->launches++;
                     h->handed[MSPAI_SOLVER_SPARSE_SMALL] = tiny;
-                    CUDA_TRY(h, mspai::launch_sparse_solve(8, mspai::SparseLaunch::kTiny,
-                                                           kSparseTinySlot, pb, out, tl, nullptr,
-                                                           tiny, sc + 7, rest, rc3, st));
-                    flist = rest;
-                    fcount = rc3;
+                    CUDA_TRY(h, mspai::launch_sparse_solve(
+                                    8, mspai::SparseLaunch::kTiny, kSparseTinySlot, kSparseTinySlot,
+                                    pb, out, more(2), nullptr, tiny, sc + 7, refused, refused, st));
                 }
+                flist = refused.list;
+                fcount = refused.count;
             }
             h->launches++;
             if (fcount)
@@ -1408,7 +1414,7 @@ extern "C" int mspai_adjoint_weighted(mspai_handle* h, const mspai_csc* C, const
     CUDA_TRY(h, cudaMemsetAsync(dcnt, 0, 64 * sizeof(int32_t), st));
     CUDA_TRY(h, h->E.ensure(sizeof(int32_t) * std::max(nprob, 1)));
     CUDA_TRY(h, h->nk.ensure(sizeof(int32_t) * std::max(nprob, 1)));
-    CUDA_TRY(h, h->lists.ensure(sizeof(int32_t) * 3 * static_cast<size_t>(std::max(nprob, 1))));
+    CUDA_TRY(h, h->lists.ensure(sizeof(int32_t) * 4 * static_cast<size_t>(std::max(nprob, 1))));
     h->launches++;
     CUDA_TRY(h, mspai::launch_adjoint_plan(pb.cptr, io.mptr, io.midx, nprob, bs,
                                            h->E.as<int32_t>(), h->nk.as<int32_t>(), st));
@@ -1444,16 +1450,15 @@ extern "C" int mspai_adjoint_weighted(mspai_handle* h, const mspai_csc* C, const
         pm.pptr = io.mptr;
         pm.pidx = io.midx;
         int32_t* lists = h->lists.as<int32_t>();
-        int32_t* const rest[2] = {lists + static_cast<size_t>(nprob),
-                                  lists + 2 * static_cast<size_t>(nprob)};
-        int32_t *left = nullptr, *left_count = nullptr;
+        int32_t* const rest[3] = {lists + static_cast<size_t>(nprob),
+                                  lists + 2 * static_cast<size_t>(nprob),
+                                  lists + 3 * static_cast<size_t>(nprob)};
         h->launches += 3;
-        CUDA_TRY(h, mspai::launch_adjoint_sparse(pm, io, alist, acount, rest, dcnt + 32, &left,
-                                                 &left_count, st));
-        CUDA_TRY(h, cudaMemcpyAsync(&acount, left_count, sizeof(int32_t), cudaMemcpyDeviceToHost,
+        CUDA_TRY(h, mspai::launch_adjoint_sparse(pm, io, alist, acount, rest, dcnt + 32, st));
+        CUDA_TRY(h, cudaMemcpyAsync(&acount, dcnt + 32, sizeof(int32_t), cudaMemcpyDeviceToHost,
                                     st));
         CUDA_TRY(h, cudaStreamSynchronize(st));
-        alist = left;
+        alist = rest[0];
     }
     if (acount > 0) {
         Caps cap{};

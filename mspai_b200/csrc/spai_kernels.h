@@ -110,19 +110,25 @@ constexpr int kSmallN = 8;
 constexpr int kSmallE = 64;
 cudaError_t launch_small_qr(const Problem& pb, const Output& out, const int32_t* list, int count,
                             int32_t* rest, int32_t* rest_count, cudaStream_t st);
+// A work list in device memory that columns are appended to.
+struct WorkList {
+    int32_t* list;
+    int32_t* count;
+};
 // Solvers on the sparse normal equations (fixed_cg.cu), a CTA per column in
-// slot_bytes of shared memory; the columns that one does not take go to
-// ovf_list / *ovf_count (appended).  nnz(C) < 2^32.
+// slot_bytes of shared memory.  The columns that do not fit the slot go to
+// `larger`; to `refused` those that no slot up to `widest` bytes would take.
+// nnz(C) < 2^32.
 enum class SparseLaunch {
     kTiny,    // a warp per column, |J| <= 36, FP64
     kNarrow,  // four warps, |J| <= 144
     kMiddle,  // four warps, |J| <= 272
     kWide     // four warps, |J| <= 400
 };
-cudaError_t launch_sparse_solve(int elem_bytes, SparseLaunch kind, int slot_bytes,
+cudaError_t launch_sparse_solve(int elem_bytes, SparseLaunch kind, int slot_bytes, int widest,
                                 const Problem& pb, const Output& out, const int32_t* list,
                                 const int32_t* count_dev, int count_host, int32_t* counter,
-                                int32_t* ovf_list, int32_t* ovf_count, cudaStream_t st);
+                                const WorkList& larger, const WorkList& refused, cudaStream_t st);
 // Block columns at their start pattern (block_solve.cu); rest[0] / counts[2]: the
 // columns left to the general solver (with pattern updates also those whose
 // residual is above the tolerance).  rest: two lists of count entries;
@@ -192,11 +198,11 @@ size_t adjoint_scratch_bytes(const Caps& cap, int n, bool warp);
 cudaError_t launch_adjoint_small(const Problem& pb, const AdjointIO& io, const int32_t* list,
                                  int count, cudaStream_t st);
 // scalar columns on the sparse form of their problem (adjoint_sparse.cu; pb with
-// the result's pattern as P); what it leaves is *left[0 .. **left_count).  rest:
-// two lists of count entries; counts[6] (zero).  nnz(C) < 2^32.
+// the result's pattern as P); what it leaves is rest[0][0 .. counts[0]).  rest:
+// three lists of count entries; counts[6] (zero).  nnz(C) < 2^32.
 cudaError_t launch_adjoint_sparse(const Problem& pb, const AdjointIO& io, const int32_t* list,
-                                  int count, int32_t* const rest[2], int32_t* counts,
-                                  int32_t** left, int32_t** left_count, cudaStream_t st);
+                                  int count, int32_t* const rest[3], int32_t* counts,
+                                  cudaStream_t st);
 // *total = sum of v[0 .. n), compensated, in a fixed order; tmp: kLossParts pairs
 constexpr int kLossParts = 1024;
 cudaError_t launch_loss_sum(const double* v, int n, double* tmp, double* total, cudaStream_t st);

@@ -1,0 +1,132 @@
+"""What becomes of the columns that a solver does not take: which solvers they
+come to (Handle.solver_columns), and their values against the oracle or a dense
+computation in numpy.  Tolerances per entry as for every column: 1e-8 in mixed
+mode, 1e-10 in FP64 (helpers.max_rel_diff)."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+import mspai_b200 as mb
+from helpers import max_rel_diff, same_pattern
+from oracle import pyoracle as O
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"fp64": 1e-10, "mixed": 1e-8}
+SPARSE = ("sparse_25k", "sparse_42k", "sparse_104k")
+
+
+@pytest.fixture
+def h():
+    handle = mb.Handle(0)
+    yield handle
+    handle.close()
+
+
+def matrix(n, per_col, dominance, seed):
+    """per_col random off-diagonal entries a column, diagonal `dominance` times
+    their absolute sum."""
+    rng = np.random.default_rng(seed)
+    rows = np.concatenate([rng.choice(n, per_col, replace=False) for _ in range(n)])
+    cols = np.repeat(np.arange(n), per_col)
+    A = sp.csc_matrix((rng.standard_normal(rows.size), (rows, cols)), shape=(n, n))
+    A.setdiag(0.0)
+    A.eliminate_zeros()
+    A = sp.csc_matrix(A + sp.diags(dominance * np.asarray(abs(A).sum(axis=0)).ravel() + 0.1))
+    A.sort_indices()
+    return A
+
+
+def pattern(n, sizes, seed):
+    rng = np.random.default_rng(seed)
+    rows, cols = [], []
+    for k in range(n):
+        s = sizes[k % len(sizes)]
+        J = np.sort(np.append(rng.choice(np.delete(np.arange(n), k), s - 1, replace=False), k))
+        rows += J.tolist()
+        cols += [k] * s
+    return sp.csc_matrix((np.ones(len(rows)), (rows, cols)), shape=(n, n))
+
+
+def column(M, k):
+    return M.indices[M.indptr[k]:M.indptr[k + 1]]
+
+
+def spectral_radius(A, J):
+    """Of D^-1/2 |G - D| D^-1/2, G = A_J^T A_J: no certificate above 0.9."""
+    X = np.abs(A[:, J].toarray())
+    X /= np.sqrt((X ** 2).sum(axis=0))
+    return np.linalg.eigvalsh(X.T @ X)[-1] - 1.0
+
+
+def check(h, A, P, prec):
+    M = h.result()
+    res, _, status = h.column_info()
+    o = O.spai_scalar(A, P, ns=0)
+    assert np.all(status == 0)
+    assert same_pattern(M, o.M)
+    assert max_rel_diff(M, o.M) < TOL[prec]
+    assert np.allclose(res, o.res, rtol=1e-9, atol=1e-13)
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+def test_no_certificate_means_the_dense_solver_at_once(h, prec):
+    n = 250
+    A = matrix(n, 10, 0.2, seed=2)
+    P = pattern(n, (40, 55), seed=3)
+    for k in range(n):
+        assert spectral_radius(A, column(P, k)) > 0.95
+    for _ in range(2):
+        h.setup(A, P, options=mb.Options(ns=0, prec=prec))
+        c = h.solver_columns()
+        assert [c[s] for s in SPARSE] == [n, 0, 0]
+        assert c["fixed"] == n
+    check(h, A, P, prec)
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+def test_only_columns_that_do_not_fit_go_to_the_next_slot(h, prec):
+    """Certified columns of up to 144, 272 and 400 unknowns, and larger ones:
+    those fit no slot."""
+    n, sizes = 1200, (60, 120, 200, 380, 410)
+    A = matrix(n, 3, 30.0, seed=4)
+    P = pattern(n, sizes, seed=5)
+    h.setup(A, P, options=mb.Options(ns=0, prec=prec))
+    c = h.solver_columns()
+    assert [c[s] for s in SPARSE] == [n, 2 * n // 5, n // 5]
+    assert c["fixed"] == n // 5
+    check(h, A, P, prec)
+    M0 = h.result()
+    h.setup(A, P, options=mb.Options(ns=0, prec=prec))
+    assert np.array_equal(M0.data, h.result().data)
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+@pytest.mark.parametrize("keep", [False, True])
+def test_gradient_of_columns_without_certificate(h, prec, keep):
+    """gbar . M at columns that the adjoint's iteration refuses (with and without
+    a kept factor), and at certified ones, against lambda from numpy."""
+    n = 200
+    A = matrix(n, 6, 0.8, seed=6)
+    P = pattern(n, (40, 60), seed=7)
+    rho = np.array([spectral_radius(A, column(P, k)) for k in range(n)])
+    assert np.any(rho > 0.95) and np.any(rho < 0.8)
+    gbar = np.random.default_rng(8).standard_normal(P.nnz)
+    h.setup(A, P, options=mb.Options(ns=0, prec=prec, keep_factors=keep))
+    dC, _, loss = h.adjoint(A, None, gbar=gbar, residual_weight=0.0)
+    D = A.toarray()
+    g = np.zeros_like(D)
+    value = 0.0
+    for k in range(n):
+        J = column(P, k)
+        gb = gbar[P.indptr[k]:P.indptr[k + 1]]
+        CJ = D[:, J]
+        e = np.zeros(n)
+        e[k] = 1.0
+        m = np.linalg.lstsq(CJ, e, rcond=None)[0]
+        lam = np.linalg.solve(CJ.T @ CJ, gb)
+        g[:, J] += np.outer(e - CJ @ m, lam) - np.outer(CJ @ lam, m)
+        value += gb @ m
+    ref = g[A.indices, np.repeat(np.arange(n), np.diff(A.indptr))]
+    assert np.max(np.abs(dC - ref)) <= TOL[prec] * np.max(np.abs(ref))
+    assert abs(loss - value) <= TOL[prec] * np.sqrt(n) * abs(value)
