@@ -10,7 +10,11 @@
 namespace mspai {
 
 // Solves column `col`; nothing of it is written unless it is taken (uniformly).
-template <class T, int NW, int K>
+// AGAIN: a re-setup, which starts from M's previous values; a column that is too
+// far from them is left to the launches without.  (Kernels of their own: at 64
+// registers a thread the choice costs the other setups 2 % of their time, and a
+// second start in the same kernel the re-setups 1.5 %.)
+template <class T, int NW, int K, bool AGAIN>
 __device__ Taken sparse_column(CgShared& sh, const Problem& pb, const Output& out, int col,
                                char* base, int cap, int widest)
 {
@@ -28,13 +32,12 @@ __device__ Taken sparse_column(CgShared& sh, const Problem& pb, const Output& ou
                                                                                  : Taken::kNo;
     }
     else {
-        // a re-setup starts from M's previous values
-        const double* prev = out.reuse_steps > 0 ? out.oval + g.p0 : nullptr;
-        const int steps = cg_solve<T, NW, K>(sh, parity, g, at, nlong, nullptr, prev);
+        const int steps = cg_solve<T, NW, K>(sh, parity, g, at, nlong, nullptr,
+                                             AGAIN ? out.oval + g.p0 : nullptr);
         if (steps < 0)
-            return Taken::kNo;
+            return AGAIN && steps == -2 ? Taken::kFar : Taken::kNo;
         write_column<NW, K>(sh, parity, g, out, col, at, steps * (4.0 * g.ns + 6.0 * g.n));
-        if (prev && threadIdx.x == 0)
+        if (AGAIN && threadIdx.x == 0)
             atomicAdd(out.reuse_count, 1);
         return Taken::kYes;
     }
@@ -42,12 +45,12 @@ __device__ Taken sparse_column(CgShared& sh, const Problem& pb, const Output& ou
 
 namespace {
 
-template <class T, int NW, int K, int MINB>
+template <class T, int NW, int K, int MINB, bool AGAIN>
 __global__ void __launch_bounds__(32 * NW, MINB)
     sparse_solve_kernel(Problem pb, Output out, const int32_t* __restrict__ list,
                         const int32_t* __restrict__ count_dev, int count_host,
                         int32_t* __restrict__ counter, WorkList larger, WorkList refused,
-                        int slot_bytes, int widest)
+                        WorkList far, int slot_bytes, int widest)
 {
     extern __shared__ __align__(16) char smem[];
     __shared__ CgShared sh;
@@ -61,21 +64,23 @@ __global__ void __launch_bounds__(32 * NW, MINB)
         if (t >= count)
             break;
         const int col = list[t];
-        const Taken taken = sparse_column<T, NW, K>(sh, pb, out, col, smem, slot_bytes, widest);
+        const Taken taken =
+            sparse_column<T, NW, K, AGAIN>(sh, pb, out, col, smem, slot_bytes, widest);
         if (taken != Taken::kYes && threadIdx.x == 0) {
-            const WorkList& to = taken == Taken::kLarger ? larger : refused;
+            const WorkList& to =
+                taken == Taken::kLarger ? larger : (taken == Taken::kFar ? far : refused);
             to.list[atomicAdd(to.count, 1)] = col;
         }
     }
 }
 
-template <class T, int NW, int K, int MINB>
+template <class T, int NW, int K, int MINB, bool AGAIN>
 cudaError_t launch_sparse_t(int slot_bytes, int widest, const Problem& pb, const Output& out,
                             const int32_t* list, const int32_t* count_dev, int count_host,
                             int32_t* counter, const WorkList& larger, const WorkList& refused,
-                            cudaStream_t st)
+                            const WorkList& far, cudaStream_t st)
 {
-    auto kern = sparse_solve_kernel<T, NW, K, MINB>;
+    auto kern = sparse_solve_kernel<T, NW, K, MINB, AGAIN>;
     cudaError_t e =
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, slot_bytes);
     if (e != cudaSuccess)
@@ -90,8 +95,21 @@ cudaError_t launch_sparse_t(int slot_bytes, int widest, const Problem& pb, const
     if (count_dev == nullptr)
         grid = std::min(grid, std::max(count_host, 1));
     kern<<<grid, 32 * NW, slot_bytes, st>>>(pb, out, list, count_dev, count_host, counter, larger,
-                                            refused, slot_bytes, widest);
+                                            refused, far, slot_bytes, widest);
     return cudaGetLastError();
+}
+
+// The launch of a slot class; the narrow one at eight CTAs per SM in FP32, six in
+// FP64.
+template <class T, bool AGAIN>
+auto sparse_launch(SparseLaunch kind)
+{
+    auto launch = launch_sparse_t<T, 4, 2, sizeof(T) == 4 ? 8 : 6, AGAIN>;
+    if (kind == SparseLaunch::kMiddle)
+        launch = launch_sparse_t<T, 4, 3, 5, AGAIN>;
+    else if (kind == SparseLaunch::kWide)
+        launch = launch_sparse_t<T, 4, 4, 2, AGAIN>;
+    return launch;
 }
 
 }  // namespace
@@ -99,18 +117,20 @@ cudaError_t launch_sparse_t(int slot_bytes, int widest, const Problem& pb, const
 cudaError_t launch_sparse_solve(int elem_bytes, SparseLaunch kind, int slot_bytes, int widest,
                                 const Problem& pb, const Output& out, const int32_t* list,
                                 const int32_t* count_dev, int count_host, int32_t* counter,
-                                const WorkList& larger, const WorkList& refused, cudaStream_t st)
+                                const WorkList& larger, const WorkList& refused, const WorkList& far,
+                                cudaStream_t st)
 {
-    const bool f = elem_bytes == 4;
-    auto launch = launch_sparse_t<double, 1, 2, 16>;
-    if (kind == SparseLaunch::kNarrow)
-        launch = f ? launch_sparse_t<float, 4, 2, 8> : launch_sparse_t<double, 4, 2, 6>;
-    else if (kind == SparseLaunch::kMiddle)
-        launch = f ? launch_sparse_t<float, 4, 3, 5> : launch_sparse_t<double, 4, 3, 5>;
-    else if (kind == SparseLaunch::kWide)
-        launch = f ? launch_sparse_t<float, 4, 4, 2> : launch_sparse_t<double, 4, 4, 2>;
+    if (kind == SparseLaunch::kTiny)
+        return launch_sparse_t<double, 1, 2, 16, false>(slot_bytes, widest, pb, out, list,
+                                                        count_dev, count_host, counter, larger,
+                                                        refused, far, st);
+    const auto launch = far.list
+                            ? (elem_bytes == 4 ? sparse_launch<float, true>(kind)
+                                               : sparse_launch<double, true>(kind))
+                            : (elem_bytes == 4 ? sparse_launch<float, false>(kind)
+                                               : sparse_launch<double, false>(kind));
     return launch(slot_bytes, widest, pb, out, list, count_dev, count_host, counter, larger,
-                  refused, st);
+                  refused, far, st);
 }
 
 }  // namespace mspai

@@ -546,7 +546,7 @@ __device__ bool hub_solve(CgShared& sh, int& parity, const SharedEntries& g, con
 // Solves min ||C x - b|| (rhs: C^T C x = rhs) into xs; returns the steps taken,
 // -1 (uniformly) when the column is not certified or does not converge.  y
 // holds b - C x (-C x) on the shared rows.  prev: a previous solution in the
-// order of J to start from; -1 as well when its gradient is not below 1/16 of
+// order of J to start from, or null; -2 when its gradient is not below 1/16 of
 // that of x = 0 (the values have changed too much for a start from it).
 template <class T, int NW, int K>
 __device__ int cg_solve(CgShared& sh, int& parity, const SharedEntries& g, const int (&at)[K],
@@ -772,7 +772,7 @@ __device__ int cg_solve(CgShared& sh, int& parity, const SharedEntries& g, const
             if (!prev)
                 g0 = gam;
             else if (!(gam <= 0x1p-8 * g0))
-                return -1;
+                return -2;
         }
         // the gradient is 2^-52 of its first value (or zero), or below 2^-48 and
         // no longer shrinking: rounding level

@@ -142,6 +142,7 @@ struct SharedEntries {
 enum class Taken {
     kYes,
     kLarger,  // it does not fit this slot
+    kFar,     // a re-setup's column, too far from its previous solution
     kNo       // it fits no slot, or the solver refuses it: the next slot would as well
 };
 

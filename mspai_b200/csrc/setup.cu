@@ -908,9 +908,11 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             const int32_t* flist = list;
             const int32_t* fcount = nullptr;
             if (sparse) {
-                // columns for the second and the third slot, refused ones; queues
-                int32_t* sc = dcnt + 28;
-                CUDA_TRY(h, cudaMemsetAsync(sc, 0, 8 * sizeof(int32_t), st));
+                // columns for the second and the third slot, refused ones, a
+                // re-setup's far ones; four queues; the same for the first run
+                // of a re-setup
+                int32_t* sc = dcnt + 44;
+                CUDA_TRY(h, cudaMemsetAsync(sc, 0, 16 * sizeof(int32_t), st));
                 int32_t* lists = h->lists.as<int32_t>();
                 auto more = [&](int k) { return lists + static_cast<size_t>(kLists + k) * nprob; };
                 const mspai::WorkList refused{more(4), sc + 2};
@@ -921,27 +923,40 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
                     widest = c.slot_bytes;
                     classes++;
                 }
-                for (int k = 0; k < classes && hc[1] > 0; k++) {
-                    const SparseClass& c = kSparseClasses[k];
-                    const mspai::WorkList larger =
-                        k + 1 < classes ? mspai::WorkList{more(k), sc + k} : refused;
-                    h->launches++;
-                    if (fcount)
-                        h->handed_at[MSPAI_SOLVER_SPARSE_25K + k] = static_cast<int>(fcount - dcnt);
-                    else
-                        h->handed[MSPAI_SOLVER_SPARSE_25K + k] = hc[1];
-                    CUDA_TRY(h, mspai::launch_sparse_solve(elem, c.kind, c.slot_bytes, widest, pb,
-                                                           out, flist, fcount, hc[1], sc + 4 + k,
-                                                           larger, refused, st));
-                    flist = larger.list;
-                    fcount = larger.count;
+                // a re-setup runs the slots twice: from M's previous values, then
+                // from zero for the columns that are too far from these
+                const mspai::WorkList far =
+                    reuse_now ? mspai::WorkList{more(2), sc + 3} : mspai::WorkList{};
+                for (int run = reuse_now ? 0 : 1; run < 2 && hc[1] > 0; run++) {
+                    const bool first = run == 0 || !reuse_now;
+                    int32_t* const cn = sc + 8 * (1 - run);
+                    flist = first ? list : far.list;
+                    fcount = first ? nullptr : far.count;
+                    for (int k = 0; k < classes; k++) {
+                        const SparseClass& c = kSparseClasses[k];
+                        const mspai::WorkList larger =
+                            k + 1 < classes ? mspai::WorkList{more(k), cn + k} : refused;
+                        h->launches++;
+                        if (k == 0)
+                            h->handed[MSPAI_SOLVER_SPARSE_25K] = hc[1];
+                        else if (first)
+                            h->handed_at[MSPAI_SOLVER_SPARSE_25K + k] =
+                                static_cast<int>(fcount - dcnt);
+                        CUDA_TRY(h, mspai::launch_sparse_solve(
+                                        elem, c.kind, c.slot_bytes, widest, pb, out, flist, fcount,
+                                        hc[1], cn + 4 + k, larger, refused,
+                                        run == 0 ? far : mspai::WorkList{}, st));
+                        flist = larger.list;
+                        fcount = larger.count;
+                    }
                 }
                 if (tiny > 0) {
                     h->launches++;
                     h->handed[MSPAI_SOLVER_SPARSE_SMALL] = tiny;
                     CUDA_TRY(h, mspai::launch_sparse_solve(
                                     8, mspai::SparseLaunch::kTiny, kSparseTinySlot, kSparseTinySlot,
-                                    pb, out, more(2), nullptr, tiny, sc + 7, refused, refused, st));
+                                    pb, out, more(2), nullptr, tiny, sc + 7, refused, refused,
+                                    mspai::WorkList{}, st));
                 }
                 flist = refused.list;
                 fcount = refused.count;

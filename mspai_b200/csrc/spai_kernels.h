@@ -118,7 +118,8 @@ struct WorkList {
 // Solvers on the sparse normal equations (fixed_cg.cu), a CTA per column in
 // slot_bytes of shared memory.  The columns that do not fit the slot go to
 // `larger`; to `refused` those that no slot up to `widest` bytes would take.
-// nnz(C) < 2^32.
+// far: null, or (a re-setup) the columns start from M's previous values and those
+// that are too far from them go there.  nnz(C) < 2^32.
 enum class SparseLaunch {
     kTiny,    // a warp per column, |J| <= 36, FP64
     kNarrow,  // four warps, |J| <= 144
@@ -128,7 +129,8 @@ enum class SparseLaunch {
 cudaError_t launch_sparse_solve(int elem_bytes, SparseLaunch kind, int slot_bytes, int widest,
                                 const Problem& pb, const Output& out, const int32_t* list,
                                 const int32_t* count_dev, int count_host, int32_t* counter,
-                                const WorkList& larger, const WorkList& refused, cudaStream_t st);
+                                const WorkList& larger, const WorkList& refused, const WorkList& far,
+                                cudaStream_t st);
 // Block columns at their start pattern (block_solve.cu); rest[0] / counts[2]: the
 // columns left to the general solver (with pattern updates also those whose
 // residual is above the tolerance).  rest: two lists of count entries;

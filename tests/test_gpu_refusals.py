@@ -130,3 +130,31 @@ def test_gradient_of_columns_without_certificate(h, prec, keep):
     ref = g[A.indices, np.repeat(np.arange(n), np.diff(A.indptr))]
     assert np.max(np.abs(dC - ref)) <= TOL[prec] * np.max(np.abs(ref))
     assert abs(loss - value) <= TOL[prec] * np.sqrt(n) * abs(value)
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+def test_resetup_far_from_the_previous_values(h, prec):
+    """Certified columns whose values have changed too much for a start from the
+    previous solution start from zero: no dense factorization, none reused."""
+    n = 500
+    A = matrix(n, 5, 2.0, seed=9)
+    P = pattern(n, (40, 90), seed=10)
+    h.setup(A, P, options=mb.Options(ns=0, prec=prec, keep_factors=True))
+    assert h.solver_columns()["fixed"] == n  # the factors are made here
+    again = mb.Options(ns=0, prec=prec, keep_factors=True, reuse_factors=4)
+    rng = np.random.default_rng(11)
+    far = A.copy()
+    far.data = A.data * np.where(rng.random(A.nnz) < 0.5, -1.0, 1.5)
+    near = far.copy()
+    near.data = far.data * (1.0 + 1e-5 * rng.standard_normal(A.nnz))
+    for k in range(n):
+        assert max(spectral_radius(M, column(P, k)) for M in (far, near)) < 0.8
+    h.setup(far, P, options=again)
+    c = h.solver_columns()
+    assert sum(c[s] for s in SPARSE) >= n and c["fixed"] == 0
+    assert h.stats()["factor_reuse_columns"] == 0
+    check(h, far, P, prec)
+    h.setup(near, P, options=again)  # from the solution made from zero
+    assert h.solver_columns()["fixed"] == 0
+    assert h.stats()["factor_reuse_columns"] == n
+    check(h, near, P, prec)
