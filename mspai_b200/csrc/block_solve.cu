@@ -18,9 +18,10 @@
 //     x = 0 of fixed_solve.cuh, for the bs right-hand sides, with its tests; FP64
 //     mode, which has no refinement, keeps the result only when the first
 //     correction is already below 2^-44 of the solution.
-// A column that does not fit, does not converge or (pattern updates) whose
-// residual is above the tolerance goes to the general solver, so the row
-// structure that the updates need is only built when a column is left.
+// A column that does not fit goes to the next launch (more shared memory); one that
+// does not converge or (pattern updates) whose residual is above the tolerance would
+// be refused there as well and goes to the general solver at once.  The row structure
+// that the updates need is only built when a column is left.
 //   Bound: latency of the blocked Cholesky and of the triangular solves at two
 //   CTAs of 256 threads per SM (mixed), one (FP64).  8,000 block columns of a
 //   20^3 27-point stencil with 3 x 3 blocks: 36.9 ms in the general solver, 12.7 ms
@@ -53,10 +54,16 @@ __device__ __forceinline__ void load4(const double* p, double (&v)[4])
     v[3] = b.y;
 }
 
-// Solves block column kb; false (uniformly) when it is left to the general
-// solver (nothing is written then).
+// What becomes of a block column.
+enum class Fit {
+    kYes,     // solved
+    kLarger,  // it does not fit the arena
+    kNo       // left to the general solver
+};
+
+// Solves block column kb (uniformly); nothing is written unless it is taken.
 template <class T, int NT>
-__device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Problem& pb,
+__device__ Fit block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Problem& pb,
                              const Output& out, int kb, char* base, int cap)
 {
     const int tid = threadIdx.x, lane = tid & 31;
@@ -64,7 +71,7 @@ __device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Prob
     const int64_t p0 = pb.pptr[kb];
     const int n = bs * static_cast<int>(pb.pptr[kb + 1] - p0);
     if (n < 1 || n > 255)
-        return false;
+        return Fit::kNo;
     auto scol = [&](int jj) { return bs * pb.pidx[p0 + jj / bs] + jj % bs; };
     FixArena a{base, cap, 0, cap};
     int32_t* off = a.low<int32_t>(n + 1);
@@ -72,7 +79,7 @@ __device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Prob
     double* x = a.low<double>(n * bs);
     T* gv = a.low<T>(n * bs);
     if (!a.ok())
-        return false;
+        return Fit::kLarger;
     for (int jj = tid; jj < n; jj += NT) {
         const int j = scol(jj);
         cb[jj] = static_cast<uint32_t>(pb.cptr[j]);
@@ -85,7 +92,7 @@ __device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Prob
         fs.chol_fail = 0;
     }
     if (E < 1 || E > 0xffff)
-        return false;
+        return Fit::kNo;
     uint16_t* R = a.low<uint16_t>(E);  // row number of entry e
     // ---- rows: hash table of at least E / 4 (small columns: 1.5 E) slots
     const int hs = next_pow2(max(64, E <= 1024 ? E + E / 2 : E / 4));
@@ -94,7 +101,7 @@ __device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Prob
     int32_t* first = a.high<int32_t>(hs);
     int32_t* flag = a.high<int32_t>(E);
     if (!a.ok() || hs > 0x10000)
-        return false;
+        return Fit::kLarger;
     g.sync();
     for (int i = tid; i < hs; i += NT) {
         key[i] = -1;
@@ -122,7 +129,7 @@ __device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Prob
     }
     g.sync();
     if (fs.chol_fail)
-        return false;
+        return Fit::kLarger;
     for (int e = tid; e < E; e += NT)
         flag[e] = first[R[e]] == e ? 1 : 0;
     g.sync();
@@ -133,7 +140,7 @@ __device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Prob
     int32_t* rs = a.low<int32_t>(m + 1);   // starts of the rows' entries
     double* r = a.low<double>(m * bs);     // residual
     if (!a.ok())
-        return false;
+        return Fit::kLarger;
     // (a first entry's slot is overwritten by its own thread only after every
     // flag is made: the scan's barriers lie in between)
     for (int e = tid; e < E; e += NT) {
@@ -180,7 +187,7 @@ __device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Prob
     T* d = a.low<T>(max(4 * m, max(kFixPanel * n, kFixPanel * kFixPanel * nblk)));
     T* tile = d;
     if (!a.ok())
-        return false;
+        return Fit::kLarger;
     for (int jj = tid / 8; jj < n; jj += NT / 8)
         for (int e = off[jj] + (tid & 7); e < off[jj + 1]; e += 8)
             V[e] = static_cast<T>(__ldg(pb.cval + cb[jj] + (e - off[jj])));
@@ -236,7 +243,7 @@ __device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Prob
         g.sync();
     }
     if (!fix_cholesky<T, NT>(g, fs, G, n, tile, r11))
-        return false;
+        return Fit::kNo;
     T* D = tile;
     fix_invert_diag<T, NT>(G, n, D);
     for (int i = tid; i < n * bs; i += NT)
@@ -334,7 +341,7 @@ __device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Prob
     }
     const double res = sqrt(r2);
     if (!conv || (pb.ns > 0 && !(res <= pb.ep * sqrt(static_cast<double>(bs)))))
-        return false;
+        return Fit::kNo;
     // ---- the bs scalar columns of M
     for (int c = 0; c < bs; c++) {
         const int sc = bs * kb + c;
@@ -365,7 +372,7 @@ __device__ bool block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Prob
         wk[2] += 12.0 * E + 16.0 * dn + 8.0 * dm * dr;
     }
     (void)lane;
-    return true;
+    return Fit::kYes;
 }
 
 // Block columns of at most eight unknowns, FP64: eight lanes per column, four
@@ -384,7 +391,7 @@ __device__ __forceinline__ double sum8(double v)
 
 __global__ void __launch_bounds__(128)
     block_small_kernel(Problem pb, Output out, const int32_t* __restrict__ list, int count,
-                       int32_t* __restrict__ ovf_list, int32_t* __restrict__ ovf_count)
+                       WorkList larger, WorkList left)
 {
     constexpr uint32_t all = 0xffffffffu;
     const int lane = threadIdx.x & 31, grp = lane >> 3, l8 = lane & 7;
@@ -395,10 +402,12 @@ __global__ void __launch_bounds__(128)
          t0 < count; t0 += 4 * static_cast<int64_t>(warps)) {
         const int kb = t0 + grp < count ? list[t0 + grp] : -1;
         int n = 0, col = 0;
+        bool wide = false;  // more than eight unknowns
         int64_t a0 = 0, a1 = 0, q0 = 0, q1 = 0;
         if (kb >= 0) {
             const int64_t p0 = pb.pptr[kb];
             n = bs * static_cast<int>(pb.pptr[kb + 1] - p0);
+            wide = n > 8;
             if (n > 8 || n < 1) {
                 n = 0;
             }
@@ -556,8 +565,10 @@ __global__ void __launch_bounds__(128)
         entries += __shfl_xor_sync(all, entries, 4);
         entries += __shfl_xor_sync(all, entries, 2);
         entries += __shfl_xor_sync(all, entries, 1);
-        if (kb >= 0 && !live && l8 == 0)
-            ovf_list[atomicAdd(ovf_count, 1)] = kb;
+        if (kb >= 0 && !live && l8 == 0) {
+            const WorkList& to = wide ? larger : left;
+            to.list[atomicAdd(to.count, 1)] = kb;
+        }
 #pragma unroll
         for (int c = 0; c < 8; c++) {
             if (c >= bs)
@@ -596,8 +607,8 @@ template <class T, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
     block_solve_kernel(Problem pb, Output out, const int32_t* __restrict__ list,
                        const int32_t* __restrict__ count_dev, int count_host,
-                       int32_t* __restrict__ counter, int32_t* __restrict__ ovf_list,
-                       int32_t* __restrict__ ovf_count, int arena_bytes)
+                       int32_t* __restrict__ counter, WorkList larger, WorkList left,
+                       int arena_bytes)
 {
     extern __shared__ __align__(16) char smem[];
     __shared__ FixShared<T> fs;
@@ -613,15 +624,18 @@ __global__ void __launch_bounds__(NT, MINB)
         if (t >= count)
             break;
         const int kb = list[t];
-        if (!block_column<T, NT>(g, fs, pb, out, kb, smem, arena_bytes) && threadIdx.x == 0)
-            ovf_list[atomicAdd(ovf_count, 1)] = kb;
+        const Fit fit = block_column<T, NT>(g, fs, pb, out, kb, smem, arena_bytes);
+        if (fit != Fit::kYes && threadIdx.x == 0) {
+            const WorkList& to = fit == Fit::kLarger ? larger : left;
+            to.list[atomicAdd(to.count, 1)] = kb;
+        }
     }
 }
 
 template <class T, int NT, int MINB>
 cudaError_t launch_block_t(int arena, const Problem& pb, const Output& out, const int32_t* list,
                            const int32_t* count_dev, int count, int32_t* counter,
-                           int32_t* ovf_list, int32_t* ovf_count, cudaStream_t st)
+                           const WorkList& larger, const WorkList& left, cudaStream_t st)
 {
     auto kern = block_solve_kernel<T, NT, MINB>;
     cudaError_t e =
@@ -635,33 +649,33 @@ cudaError_t launch_block_t(int arena, const Problem& pb, const Output& out, cons
     if (per_sm < 1)
         return cudaErrorInvalidConfiguration;
     const int grid = std::max(1, std::min(per_sm * num_sms(), count));
-    kern<<<grid, NT, arena, st>>>(pb, out, list, count_dev, count, counter, ovf_list, ovf_count,
-                                  arena);
+    kern<<<grid, NT, arena, st>>>(pb, out, list, count_dev, count, counter, larger, left, arena);
     return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_block_solve(int elem_bytes, const Problem& pb, const Output& out,
-                               const int32_t* list, int count, int32_t* const rest[2],
+                               const int32_t* list, int count, int32_t* const rest[3],
                                int32_t* counts, cudaStream_t st)
 {
     // at most eight unknowns: eight lanes; small columns in FP64 (no refinement
     // to speak of on a few unknowns), 64 threads; then 256 threads and two CTAs
     // per SM, in FP64 one
+    const WorkList wide{rest[0], counts}, large{rest[1], counts + 1}, left{rest[2], counts + 2};
     const int blocks = std::max(1, std::min((count + 15) / 16, num_sms() * 16));
-    block_small_kernel<<<blocks, 128, 0, st>>>(pb, out, list, count, rest[0], counts);
+    block_small_kernel<<<blocks, 128, 0, st>>>(pb, out, list, count, wide, left);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
-        e = launch_block_t<double, 64, 12>(15 * 1024, pb, out, rest[0], counts, count, counts + 3,
-                                           rest[1], counts + 1, st);
+        e = launch_block_t<double, 64, 12>(15 * 1024, pb, out, wide.list, wide.count, count,
+                                           counts + 3, large, left, st);
     if (e != cudaSuccess)
         return e;
     if (elem_bytes == 4)
-        return launch_block_t<float, 256, 2>(107 * 1024, pb, out, rest[1], counts + 1, count,
-                                             counts + 4, rest[0], counts + 2, st);
-    return launch_block_t<double, 256, 1>(212 * 1024, pb, out, rest[1], counts + 1, count,
-                                          counts + 4, rest[0], counts + 2, st);
+        return launch_block_t<float, 256, 2>(107 * 1024, pb, out, large.list, large.count, count,
+                                             counts + 4, left, left, st);
+    return launch_block_t<double, 256, 1>(212 * 1024, pb, out, large.list, large.count, count,
+                                          counts + 4, left, left, st);
 }
 
 }  // namespace mspai

@@ -806,8 +806,9 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
         int left = count;  // columns for the solver below
         if (blocks) {
             int32_t* lists = h->lists.as<int32_t>();
-            int32_t* const rest[2] = {lists + static_cast<size_t>(kLists) * nprob,
-                                      lists + static_cast<size_t>(kLists + 1) * nprob};
+            int32_t* const rest[3] = {lists + static_cast<size_t>(kLists) * nprob,
+                                      lists + static_cast<size_t>(kLists + 1) * nprob,
+                                      lists + static_cast<size_t>(kLists + 2) * nprob};
             int32_t* bc = dcnt + 28;
             CUDA_TRY(h, cudaMemsetAsync(bc, 0, 5 * sizeof(int32_t), st));
             CUDA_TRY(h, cudaEventRecord(h->evb[2 * b], st));
@@ -824,7 +825,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             CUDA_TRY(h, cudaStreamSynchronize(st));
             if (left == 0)
                 continue;
-            list = rest[0];
+            list = rest[2];
             if (need_rows) {
                 if ((rc = build_rows()) != MSPAI_OK)
                     return rc;

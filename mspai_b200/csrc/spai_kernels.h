@@ -131,12 +131,13 @@ cudaError_t launch_sparse_solve(int elem_bytes, SparseLaunch kind, int slot_byte
                                 const int32_t* count_dev, int count_host, int32_t* counter,
                                 const WorkList& larger, const WorkList& refused, const WorkList& far,
                                 cudaStream_t st);
-// Block columns at their start pattern (block_solve.cu); rest[0] / counts[2]: the
+// Block columns at their start pattern (block_solve.cu); rest[2] / counts[2]: the
 // columns left to the general solver (with pattern updates also those whose
-// residual is above the tolerance).  rest: two lists of count entries;
-// counts[5] (zero).  nnz(C) < 2^32.
+// residual is above the tolerance).  counts[0], counts[1]: those of more than eight
+// unknowns, and of these those that the second launch does not hold.  rest: three
+// lists of count entries; counts[5] (zero).  nnz(C) < 2^32.
 cudaError_t launch_block_solve(int elem_bytes, const Problem& pb, const Output& out,
-                               const int32_t* list, int count, int32_t* const rest[2],
+                               const int32_t* list, int count, int32_t* const rest[3],
                                int32_t* counts, cudaStream_t st);
 cudaError_t launch_scan_lengths(const int32_t* len, int n, int64_t* ptr, int64_t* tmp,
                                 cudaStream_t st);

@@ -158,3 +158,42 @@ def test_resetup_far_from_the_previous_values(h, prec):
     assert h.solver_columns()["fixed"] == 0
     assert h.stats()["factor_reuse_columns"] == n
     check(h, near, P, prec)
+
+
+def block_problem(nb, bs, blocks, seed, diag=6.0):
+    """Random block matrix, four block entries a block column, and a block pattern
+    of `blocks` blocks a column."""
+    rng = np.random.default_rng(seed)
+    J = lambda m: [sorted({k} | set(rng.choice(np.delete(np.arange(nb), k), m - 1,
+                                               replace=False).tolist())) for k in range(nb)]
+    A = np.zeros((bs * nb, bs * nb))
+    for k, rows in enumerate(J(4)):
+        for b in rows:
+            A[bs * b:bs * b + bs, bs * k:bs * k + bs] = rng.standard_normal((bs, bs))
+    A = sp.csc_matrix(A + diag * np.eye(bs * nb))
+    A.sort_indices()
+    rows = J(blocks)
+    P = sp.csc_matrix((np.ones(blocks * nb), np.concatenate(rows),
+                       np.arange(nb + 1) * blocks), shape=(nb, nb))
+    return A, P
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+@pytest.mark.parametrize("bs,blocks,solver", [(3, 1, "block_small"), (3, 4, "block_64"),
+                                              (2, 20, "block_256")])
+def test_block_columns_above_the_tolerance(h, prec, bs, blocks, solver):
+    """A block column that is solved at its start pattern and needs an update comes
+    to no other solver of the start pattern."""
+    nb = 60
+    A, P = block_problem(nb, bs, blocks, seed=blocks)
+    h.setup(A, P, options=mb.Options(ns=1, mn=2, ep=1e-3, bs=bs, prec=prec))
+    c = h.solver_columns()
+    after = {"block_small": ("block_64", "block_256"), "block_64": ("block_256",),
+             "block_256": ()}[solver]
+    assert c[solver] == nb and c["general"] == nb
+    assert all(c[s] == 0 for s in after)
+    o = O.spai_block(A, P, bs, ns=1, mn=2, ep=1e-3)
+    M = h.result()
+    assert same_pattern(M, o.M)
+    assert max_rel_diff(M, o.M) < TOL[prec]
+
