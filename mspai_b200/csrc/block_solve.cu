@@ -489,9 +489,11 @@ __global__ void __launch_bounds__(128)
                         break;
                     const double piv = __shfl_sync(all, G[k], k, 8);
                     const bool in = k < n;
-                    if (in && !(piv > 0.0))
+                    // (an infinite pivot would give x = 0 and pass for converged)
+                    const bool pos = piv > 0.0 && isfinite(piv);
+                    if (in && !pos)
                         done = true, live = false;
-                    const double inv = in && piv > 0.0 ? 1.0 / sqrt(piv) : 0.0;
+                    const double inv = in && pos ? 1.0 / sqrt(piv) : 0.0;
                     if (l8 == k)
                         linv = inv;
                     const double l = l8 > k ? G[k] * inv : 0.0;

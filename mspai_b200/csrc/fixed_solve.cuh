@@ -744,7 +744,8 @@ __device__ __forceinline__ bool fix_chol_diag(T* R, int n, int c0, int nb, int l
     for (int k = 0; k < kFixPanel; k++) {
         if (k < nb) {
             const T piv = __shfl_sync(0xffffffffu, a[k], k);
-            bad = bad || !(piv > T(0));
+            // an infinite pivot (G has overflowed) would give x = 0 and pass for converged
+            bad = bad || !(piv > T(0)) || !isfinite(piv);
             const T rkk = bad ? T(1) : sqrt(piv);
             const T inv = T(1) / rkk;
             if (lane == k) {
@@ -789,7 +790,7 @@ __device__ __forceinline__ bool fix_chol_diag(T* R, int n, int c0, int nb, int l
 // the diagonal factorization off the critical path while the trailing
 // triangle is large.  Every element of G sees the same operations in the same
 // order as in the plain right-looking order.  Returns false (uniformly) when
-// a pivot is not positive (G not numerically positive definite in T).
+// a pivot is not positive (G not numerically positive definite in T) or not finite.
 // tile: 16 n elements, 16-byte aligned (the block row of R right of the
 // diagonal block, 16 consecutive values per column); r11: 256 elements,
 // 16-byte aligned (the current diagonal block of R, dense).

@@ -197,3 +197,31 @@ def test_block_columns_above_the_tolerance(h, prec, bs, blocks, solver):
     assert same_pattern(M, o.M)
     assert max_rel_diff(M, o.M) < TOL[prec]
 
+
+
+@pytest.mark.parametrize("prec,powers", [("fp64", range(507, 513)), ("mixed", range(58, 64))])
+@pytest.mark.parametrize("bs,blocks,keep", [(3, 1, False), (3, 4, False), (3, 14, False),
+                                            (1, 50, True)])
+def test_normal_matrix_that_overflows(h, prec, powers, bs, blocks, keep):
+    """C times powers of two around the one where the squares overflow (FP64, or
+    the FP32 of the mixed mode's larger columns): a column is flagged, or it is M
+    times the inverse power."""
+    nb = 60
+    if bs > 1:
+        A, P = block_problem(nb, bs, blocks, seed=blocks)
+    else:
+        A, P = matrix(nb * 3, 6, 3.0, seed=1), pattern(nb * 3, (blocks,), seed=2)
+    o = mb.Options(ns=0, bs=bs, prec=prec, keep_factors=keep)
+    h.setup(A, P, options=o)
+    M0 = h.result()
+    S = A.copy()
+    for power in powers:
+        S.data = np.ldexp(A.data, power)
+        h.setup(S, P, options=o)
+        M = h.result()
+        _, _, status = h.column_info()
+        assert same_pattern(M, M0)
+        for k in np.flatnonzero(status == 0):
+            a, b = M0.indptr[k], M0.indptr[k + 1]
+            assert np.allclose(np.ldexp(M.data[a:b], power), M0.data[a:b], rtol=0,
+                               atol=TOL[prec] * np.max(np.abs(M0.data[a:b])))
