@@ -90,12 +90,23 @@ __device__ Fit block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Probl
     if (tid == 0) {
         off[n] = E;
         fs.chol_fail = 0;
+        fs.mcount = 0;
     }
     if (E < 1 || E > 0xffff)
         return Fit::kNo;
     uint16_t* R = a.low<uint16_t>(E);  // row number of entry e
-    // ---- rows: hash table of at least E / 4 (small columns: 1.5 E) slots
-    const int hs = next_pow2(max(64, E <= 1024 ? E + E / 2 : E / 4));
+    // ---- rows: a hash table of 1.25 times the rows that the arena can hold (what
+    // every entry and every row takes below), or of 1.5 E slots.  A column with more
+    // rows than that ends here: its insertion stops at the first row too many, so
+    // that at most one more a thread is inserted and a probe meets a free slot.
+    const int room = cap - a.lo - E * (5 + static_cast<int>(sizeof(T))) -
+                     fix_rs(n, n) * static_cast<int>(sizeof(T));
+    const int most_rows = min(E, room / (8 + 8 * bs + 4 * static_cast<int>(sizeof(T))));
+    if (most_rows < 1)
+        return Fit::kLarger;
+    const bool limited = most_rows < E;
+    const int hs = next_pow2(max(64, limited ? min(E + E / 2, most_rows + most_rows / 4 + NT)
+                                             : E + E / 2));
     const int hbits = 31 - __clz(hs);
     int32_t* key = a.high<int32_t>(hs);
     int32_t* first = a.high<int32_t>(hs);
@@ -108,27 +119,25 @@ __device__ Fit block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Probl
         first[i] = 0x7fffffff;
     }
     g.sync();
+    const volatile int* rows = &fs.mcount;
     for (int jj = tid / 8; jj < n; jj += NT / 8) {
         const int o = off[jj], len = off[jj + 1] - o;
-        for (int q = tid & 7; q < len; q += 8) {
+        for (int q = tid & 7; q < len && (!limited || *rows <= most_rows); q += 8) {
             const int row = __ldg(pb.cidx + cb[jj] + q);
             uint32_t s = (static_cast<uint32_t>(row) * 2654435761u) >> (32 - hbits);
-            int probe = 0;
-            for (; probe < hs; probe++) {
-                const int old = atomicCAS(&key[s], -1, row);
-                if (old == -1 || old == row)
-                    break;
+            int old = atomicCAS(&key[s], -1, row);
+            while (old != -1 && old != row) {
                 s = (s + 1) & (hs - 1);
+                old = atomicCAS(&key[s], -1, row);
             }
-            if (probe == hs)
-                fs.chol_fail = 1;  // more rows than slots
-            else
-                atomicMin(&first[s], o + q);
+            if (limited && old == -1)
+                atomicAdd(&fs.mcount, 1);
+            atomicMin(&first[s], o + q);
             R[o + q] = static_cast<uint16_t>(s);
         }
     }
     g.sync();
-    if (fs.chol_fail)
+    if (limited && fs.mcount > most_rows)
         return Fit::kLarger;
     for (int e = tid; e < E; e += NT)
         flag[e] = first[R[e]] == e ? 1 : 0;
@@ -567,10 +576,10 @@ __global__ void __launch_bounds__(128)
         entries += __shfl_xor_sync(all, entries, 4);
         entries += __shfl_xor_sync(all, entries, 2);
         entries += __shfl_xor_sync(all, entries, 1);
-        if (kb >= 0 && !live && l8 == 0) {
-            const WorkList& to = wide ? larger : left;
-            to.list[atomicAdd(to.count, 1)] = kb;
-        }
+        if (wide && l8 == 0)
+            larger.list[atomicAdd(larger.count, 1)] = kb;
+        else if (kb >= 0 && !live && l8 == 0)
+            left.list[atomicAdd(left.count, 1)] = kb;
 #pragma unroll
         for (int c = 0; c < 8; c++) {
             if (c >= bs)

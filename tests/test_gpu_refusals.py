@@ -225,3 +225,50 @@ def test_normal_matrix_that_overflows(h, prec, powers, bs, blocks, keep):
             a, b = M0.indptr[k], M0.indptr[k + 1]
             assert np.allclose(np.ldexp(M.data[a:b], power), M0.data[a:b], rtol=0,
                                atol=TOL[prec] * np.max(np.abs(M0.data[a:b])))
+
+
+def scattered_blocks(nb, bs, per_col, blocks, seed):
+    """Columns of per_col random entries and a strong diagonal, a random block
+    pattern: nearly every row of C(:, J) has one entry."""
+    rng = np.random.default_rng(seed)
+    n = nb * bs
+    A = matrix(n, per_col, 0.0, seed) + 3.0 * np.sqrt(per_col) * sp.identity(n)
+    A = sp.csc_matrix(A)
+    A.sort_indices()
+    rows = [np.sort(np.append(rng.choice(np.delete(np.arange(nb), k), blocks - 1, replace=False),
+                              k)) for k in range(nb)]
+    P = sp.csc_matrix((np.ones(nb * blocks), np.concatenate(rows), np.arange(nb + 1) * blocks),
+                      shape=(nb, nb))
+    return A, P
+
+
+@pytest.mark.parametrize("prec", ["mixed", "fp64"])
+@pytest.mark.parametrize("bs,per_col,blocks", [(2, 25, 20), (2, 27, 20),  # 1,024 entries, more
+                                               (2, 60, 20), (2, 100, 50), (3, 40, 8)])
+def test_block_columns_of_more_rows_than_the_arena_holds(h, prec, bs, per_col, blocks):
+    nb = 1500
+    A, P = scattered_blocks(nb, bs, per_col, blocks, seed=per_col)
+    cols = np.arange(0, nb, nb // 12)
+    h.setup(A, P, options=mb.Options(ns=0, bs=bs, prec=prec))
+    M = h.result()
+    D = A.toarray()
+    for k in cols:
+        J = (bs * column(P, k)[:, None] + np.arange(bs)).ravel()
+        x = np.linalg.lstsq(D[:, J], np.eye(nb * bs)[:, bs * k:bs * k + bs], rcond=None)[0]
+        got = M[:, bs * k:bs * k + bs].toarray()
+        assert np.allclose(got[J], x, rtol=0, atol=TOL[prec] * np.max(np.abs(x)))
+
+
+def test_block_columns_of_many_rows_are_given_up_early(h):
+    """A column with far more rows than the arena holds costs little beside its
+    solution by the general solver (a setup without refinement uses that alone):
+    before its row table stopped at the first row too many it took 4.5 times that."""
+    A, P = scattered_blocks(4000, 2, 60, 20, seed=9)
+    ms = {}
+    for refine in (0, 4):
+        o = mb.Options(ns=0, bs=2, prec="mixed", refine=refine)
+        h.setup(A, P, options=o)
+        h.setup(A, P, options=o)
+        ms[refine] = h.stats()["setup_ms"]
+    assert h.solver_columns()["general"] == 4000
+    assert ms[4] < 2.0 * ms[0]
