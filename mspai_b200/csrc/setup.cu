@@ -693,7 +693,7 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
     // fixed scalar patterns: every column beyond the warp bucket goes to the
     // fixed-pattern solver (bucket 1), which sizes its arrays per column
     const bool use_fixed = !adaptive && bs == 1 && prm->batched && !pb.qru;
-    rule.smem_w_bytes = (use_fixed || blocks) ? (int64_t(1) << 62) : h->w_smem_bytes;
+    rule.smem_w_bytes = use_fixed ? (int64_t(1) << 62) : h->w_smem_bytes;
     // the smallest fixed columns: eight lanes each (the store of R holds one
     // element type, the small QR is FP64: not when R is kept)
     const bool small = use_fixed && !out.rstore;
@@ -803,6 +803,10 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
         int32_t* list = h->lists.as<int32_t>() + static_cast<size_t>(b) * nprob;
         int32_t* counter = dcnt + 12 + b;
         CUDA_TRY(h, cudaMemsetAsync(counter, 0, sizeof(int32_t), st));
+        // small problems in mixed mode: FP64 without refinement (not when R
+        // is kept: its store has one element type)
+        const bool fp64_bucket = mixed && !out.rstore && cap.nmax <= kMixedFp64MaxN;
+        const int elem_b = fp64_bucket ? 8 : elem;
         int left = count;  // columns for the solver below
         if (blocks) {
             int32_t* lists = h->lists.as<int32_t>();
@@ -813,21 +817,22 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             CUDA_TRY(h, cudaMemsetAsync(bc, 0, 5 * sizeof(int32_t), st));
             CUDA_TRY(h, cudaEventRecord(h->evb[2 * b], st));
             h->launches += 3;
-            h->handed[MSPAI_SOLVER_BLOCK_SMALL] = count;
-            h->handed_at[MSPAI_SOLVER_BLOCK_64] = static_cast<int>(bc - dcnt);
-            h->handed_at[MSPAI_SOLVER_BLOCK_256] = static_cast<int>(bc + 1 - dcnt);
-            CUDA_TRY(h, mspai::launch_block_solve(elem, pb, out, list, count, rest, bc, st));
+            CUDA_TRY(h, mspai::launch_block_solve(elem_b, pb, out, list, count, rest, bc, st));
             CUDA_TRY(h, cudaEventRecord(h->evb[2 * b + 1], st));
             timed[b] = true;
             h->stats.bucket_columns[b] = count;
-            CUDA_TRY(h, cudaMemcpyAsync(&left, bc + 2, sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                        st));
+            int32_t ho[3] = {0, 0, 0};
+            CUDA_TRY(h, cudaMemcpyAsync(ho, bc, sizeof(ho), cudaMemcpyDeviceToHost, st));
             CUDA_TRY(h, cudaStreamSynchronize(st));
+            h->handed[MSPAI_SOLVER_BLOCK_SMALL] += count;
+            h->handed[MSPAI_SOLVER_BLOCK_64] += ho[0];
+            h->handed[MSPAI_SOLVER_BLOCK_256] += ho[1];
+            left = ho[2];
             if (left == 0)
                 continue;
             list = rest[2];
             if (need_rows) {
-                if ((rc = build_rows()) != MSPAI_OK)
+                if (!pb.rptr && (rc = build_rows()) != MSPAI_OK)
                     return rc;
                 cap.cmax = static_cast<int>(std::min<int64_t>(
                     nprob, static_cast<int64_t>(cap.emax + 1) * bs * std::max(1, max_row_nnz)));
@@ -835,10 +840,6 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
             }
         }
         int grid = 0;
-        // small problems in mixed mode: FP64 without refinement (not when R
-        // is kept: its store has one element type)
-        const bool fp64_bucket = mixed && !out.rstore && cap.nmax <= kMixedFp64MaxN;
-        const int elem_b = fp64_bucket ? 8 : elem;
         Problem pbb = pb;
         if (fp64_bucket)
             pbb.refine = 0;

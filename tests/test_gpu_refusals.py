@@ -272,3 +272,25 @@ def test_block_columns_of_many_rows_are_given_up_early(h):
         ms[refine] = h.stats()["setup_ms"]
     assert h.solver_columns()["general"] == 4000
     assert ms[4] < 2.0 * ms[0]
+
+
+def test_small_block_columns_beside_large_ones_in_fp64(h):
+    """Mixed mode solves a bucket of at most 32 unknowns a column in FP64, whatever
+    the other bucket holds: nearly dependent columns (a relative 1e-8) that the
+    normal equations refuse, 18 unknowns, beside columns of 120.  The residual of
+    a backward stable solution is the smallest one up to 1e-16 times a modest
+    factor, the FP32 factor's is not."""
+    nb, bs = 60, 3
+    A, _ = block_problem(nb, bs, 1, seed=5)
+    A = A.toarray()
+    rng = np.random.default_rng(6)
+    A[:, 1::3] = A[:, 0::3] * (1.0 + 1e-8 * rng.standard_normal(A[:, 0::3].shape))
+    A = sp.csc_matrix(A)
+    A.sort_indices()
+    P = pattern(nb, (40,) + (6,) * 9, seed=7)
+    h.setup(A, P, options=mb.Options(ns=0, bs=bs, prec="mixed"))
+    res, _, _ = h.column_info()
+    o = O.spai_block(A, P, bs, ns=0)
+    small = np.repeat(np.diff(P.indptr) == 6, bs)
+    assert h.solver_columns()["general"] >= 54
+    assert np.allclose(res[small], np.asarray(o.res).ravel()[small], rtol=1e-6, atol=1e-6)
