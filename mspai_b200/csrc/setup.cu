@@ -108,7 +108,7 @@ struct mspai_handle {
     DevBuf scratch;
     DevBuf vflag;  // device input checks
     DevBuf ax, ay; // host vectors of mspai_apply
-    DevBuf aloss, acnt;  // losses and counters of the adjoint
+    DevBuf aloss, acnt, alists;  // losses, counters and work lists of the adjoint
     // row structure of the result for mspai_apply (built on first use)
     DevBuf tptr, tcol, tval, tkeys, tperm0, tperm1, tcnt, ttemp;
     bool rows_valid = false;
@@ -286,7 +286,7 @@ void mspai_free(mspai_handle* h)
                       &h->midx, &h->mval, &h->scratch, &h->vflag, &h->ax, &h->ay,
                       &h->rkeys, &h->rslot_rep, &h->rslot_of, &h->rrep, &h->tptr, &h->tcol,
                       &h->tval, &h->tkeys, &h->tperm0, &h->tperm1, &h->tcnt, &h->ttemp,
-                      &h->rglob, &h->aloss, &h->acnt};
+                      &h->rglob, &h->aloss, &h->acnt, &h->alists};
     for (DevBuf* b : bufs)
         b->release();
     if (h->ev0)
@@ -1395,7 +1395,8 @@ extern "C" int mspai_adjoint_weighted(mspai_handle* h, const mspai_csc* C, const
     io.mval = h->res_val;
     io.wres = residual_weight;
     DevBuf gbuf, dcbuf, dbbuf;
-    // kept in the handle: the columns' losses with their sum, the counters
+    // kept in the handle: the columns' losses with their sum, the counters (and the
+    // work lists: those of the setup stay for its statistics)
     DevBuf &lossbuf = h->aloss, &cnt = h->acnt;
     if (gbar_values) {
         const double* gp = nullptr;
@@ -1431,7 +1432,7 @@ extern "C" int mspai_adjoint_weighted(mspai_handle* h, const mspai_csc* C, const
     CUDA_TRY(h, cudaMemsetAsync(dcnt, 0, 64 * sizeof(int32_t), st));
     CUDA_TRY(h, h->E.ensure(sizeof(int32_t) * std::max(nprob, 1)));
     CUDA_TRY(h, h->nk.ensure(sizeof(int32_t) * std::max(nprob, 1)));
-    CUDA_TRY(h, h->lists.ensure(sizeof(int32_t) * 4 * static_cast<size_t>(std::max(nprob, 1))));
+    CUDA_TRY(h, h->alists.ensure(sizeof(int32_t) * 4 * static_cast<size_t>(std::max(nprob, 1))));
     h->launches++;
     CUDA_TRY(h, mspai::launch_adjoint_plan(pb.cptr, io.mptr, io.midx, nprob, bs,
                                            h->E.as<int32_t>(), h->nk.as<int32_t>(), st));
@@ -1448,25 +1449,25 @@ extern "C" int mspai_adjoint_weighted(mspai_handle* h, const mspai_csc* C, const
     rule.hi = ahi;
     h->launches++;
     CUDA_TRY(h, mspai::launch_bucket(h->E.as<int32_t>(), h->nk.as<int32_t>(), nprob, rule, dcnt,
-                                     dcnt + 4, dcnt + 8, h->lists.as<int32_t>(), st));
+                                     dcnt + 4, dcnt + 8, h->alists.as<int32_t>(), st));
     int32_t hc[16];
     CUDA_TRY(h, cudaMemcpyAsync(hc, dcnt, sizeof(hc), cudaMemcpyDeviceToHost, st));
     CUDA_TRY(h, cudaStreamSynchronize(st));
     if (hc[2] > 0) {
         h->launches++;
         CUDA_TRY(h, mspai::launch_adjoint_small(
-                        pb, io, h->lists.as<int32_t>() + 2 * static_cast<size_t>(nprob), hc[2],
+                        pb, io, h->alists.as<int32_t>() + 2 * static_cast<size_t>(nprob), hc[2],
                         st));
     }
     // larger scalar columns: the sparse form of their problem; what it leaves
     // (counted on the host) goes to the general adjoint
-    const int32_t* alist = h->lists.as<int32_t>();
+    const int32_t* alist = h->alists.as<int32_t>();
     int acount = hc[0];
     if (acount > 0 && bs == 1 && C->nnz < (int64_t(1) << 32) && hc[4] > 64) {
         Problem pm = pb;
         pm.pptr = io.mptr;
         pm.pidx = io.midx;
-        int32_t* lists = h->lists.as<int32_t>();
+        int32_t* lists = h->alists.as<int32_t>();
         int32_t* const rest[3] = {lists + static_cast<size_t>(nprob),
                                   lists + 2 * static_cast<size_t>(nprob),
                                   lists + 3 * static_cast<size_t>(nprob)};
