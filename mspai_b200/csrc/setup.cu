@@ -1303,19 +1303,24 @@ int mspai_get_stats(mspai_handle* h, mspai_stats* s)
     for (int b = 0; b < 4; b++)
         h->stats.bucket_flops[b] = 0.0;
     if (h->nprob > 0 && h->lists.p) {
-        std::vector<int32_t> lists(static_cast<size_t>(kLists + kMoreLists) * h->nprob);
-        CUDA_TRY(h, cudaMemcpy(lists.data(), h->lists.p, sizeof(int32_t) * lists.size(),
-                               cudaMemcpyDeviceToHost));
         double sums[kLists] = {0.0, 0.0, 0.0, 0.0};
+        std::vector<int32_t> cols;
+        // adds the flops of the first `len` columns of work list l to bucket b's
+        auto add = [&](int l, int64_t len, int b) -> cudaError_t {
+            cols.resize(static_cast<size_t>(len));
+            if (len == 0)
+                return cudaSuccess;
+            const cudaError_t e = cudaMemcpy(
+                cols.data(), h->lists.as<int32_t>() + l * static_cast<size_t>(h->nprob),
+                sizeof(int32_t) * cols.size(), cudaMemcpyDeviceToHost);
+            for (size_t t = 0; e == cudaSuccess && t < cols.size(); t++)
+                sums[b] += work[3 * static_cast<size_t>(cols[t])];
+            return e;
+        };
         for (int b = 0; b < kLists; b++)
-            for (int64_t t = 0; t < h->list_len[b]; t++)
-                sums[b] += work[3 * static_cast<size_t>(lists[b * static_cast<size_t>(h->nprob) + t])];
-        for (int64_t t = 0; t < h->tiny_len; t++)
-            sums[1] += work[3 * static_cast<size_t>(
-                                lists[(kLists + 2) * static_cast<size_t>(h->nprob) + t])];
-        for (int64_t t = 0; t < h->small_len; t++)
-            sums[0] += work[3 * static_cast<size_t>(
-                                lists[(kLists + 3) * static_cast<size_t>(h->nprob) + t])];
+            CUDA_TRY(h, add(b, h->list_len[b], b));
+        CUDA_TRY(h, add(kLists + 2, h->tiny_len, 1));
+        CUDA_TRY(h, add(kLists + 3, h->small_len, 0));
         if (h->used_fixed) {
             h->stats.bucket_flops[0] = sums[0];
             h->stats.bucket_flops[1] = sums[1] - sums[2];
