@@ -671,14 +671,15 @@ cudaError_t launch_block_solve(int elem_bytes, const Problem& pb, const Output& 
                                int32_t* counts, cudaStream_t st)
 {
     // at most eight unknowns: eight lanes; small columns in FP64 (no refinement
-    // to speak of on a few unknowns), 64 threads; then 256 threads and two CTAs
-    // per SM, in FP64 one
+    // to speak of on a few unknowns), 64 threads and eight CTAs per SM (15 KB and
+    // the static 10 KB of shared memory); then 256 threads and two CTAs per SM, in
+    // FP64 one
     const WorkList wide{rest[0], counts}, large{rest[1], counts + 1}, left{rest[2], counts + 2};
     const int blocks = std::max(1, std::min((count + 15) / 16, num_sms() * 16));
     block_small_kernel<<<blocks, 128, 0, st>>>(pb, out, list, count, wide, left);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
-        e = launch_block_t<double, 64, 12>(15 * 1024, pb, out, wide.list, wide.count, count,
+        e = launch_block_t<double, 64, 8>(15 * 1024, pb, out, wide.list, wide.count, count,
                                            counts + 3, large, left, st);
     if (e != cudaSuccess)
         return e;

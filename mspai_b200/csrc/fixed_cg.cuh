@@ -16,7 +16,7 @@
 // level; mixed mode iterates in FP32 between restarts, as its factor is FP32 in
 // the dense path.
 //   Bound: instruction issue (0.5 to 0.6 per scheduler and cycle) and the
-//   latency of two barriers a step; a column's 20 KB of shared memory allow
+//   latency of two barriers a step; slots of 25 KB (and 1.7 KB static) allow
 //   eight CTAs per SM.  Ragged workload, 1,000,000 columns: 700 ms in the dense
 //   path, 76 ms here, 34 of them for finding and laying out the shared entries.
 //

@@ -50,7 +50,8 @@ struct SparseClass {
 constexpr SparseClass kSparseClasses[] = {{25 * 1024, mspai::SparseLaunch::kNarrow},
                                           {42 * 1024, mspai::SparseLaunch::kMiddle},
                                           {104 * 1024, mspai::SparseLaunch::kWide}};
-// Small columns: a warp each, 16 per SM (register bound).
+// Small columns: a warp each, 14 per SM (13 KB and the solver's static 1.7 KB of
+// shared memory; the registers would allow 16).
 constexpr int kSparseTinySlot = 13 * 1024;
 constexpr int kSparseTinyN = 36;
 constexpr int kSparseTinyE = 640;

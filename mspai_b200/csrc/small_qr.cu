@@ -12,8 +12,9 @@
 // registers and the group factors them by Householder reflections (dlarfg:
 // beta = -sign(alpha) ||(alpha, x)||, tau = 0 for x = 0) with three-step sums.
 // The residual is formed in FP64 from the matrix in shared memory.
-//   Bound: FP64 latency (a square root and a reciprocal per reflection) at 24
-//   warps per SM.  Anisotropic 1024^2 with two probing rows: 13.6 ms in the
+//   Bound: FP64 latency (a square root and a reciprocal per reflection) at 16
+//   warps per SM (128 registers, 38 KB of shared memory a CTA of four warps; columns
+//   of 33 to 64 rows: 8).  Anisotropic 1024^2 with two probing rows: 13.6 ms in the
 //   general warp solver, 1.6 ms here.
 #include "spai_kernels.h"
 #include "spai_solve.cuh"
