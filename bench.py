@@ -533,21 +533,30 @@ def bench_ours(args):
     kms = st["kernel_ms"][b]
     achieved = st["bucket_flops"][b] / (kms * 1e-3) / 1e12 if kms > 0 else None
     peak32 = mb.measure_fma_peak(local, fp64=False) / 1e3
+    # the fixed-pattern bucket runs the sparse solvers and, on what they refuse,
+    # the dense factorizations: named after the one that took most columns
+    came = h.solver_columns()
+    sparse = came["sparse_25k"] + came["sparse_small"]
+    kernel = ["warp_solve_kernel", "fixed_solve_kernel (first launch)",
+              "fixed_solve_kernel (large arena)", "cta_solve_kernel (fallback)"][b]
+    prof = "fixed_solve_traffic.json"
+    if b == 0 and came["small_qr"] > came["warp"]:
+        kernel = "small_qr_kernel"
+    elif b == 1 and came["fixed"] < 0.5 * sparse:
+        kernel, prof = "sparse_solve_kernel (slots of 25, 42 and 104 KB)", "sparse_solve_traffic.json"
     traffic = None
-    prof = os.path.join(HERE, "profiles", "fixed_solve_traffic.json")
+    prof = os.path.join(HERE, "profiles", prof)
     if b == 1 and os.path.exists(prof):
         try:
-            # DRAM bytes of one captured launch A of the fixed-pattern solver,
-            # scaled to this launch by the columns it solves (traffic grows
-            # with the columns processed)
+            # DRAM bytes of captured launches, scaled to these by the columns they
+            # solve (traffic grows with the columns processed)
             pj = json.load(open(prof))
             traffic = pj["dram_bytes_per_column"] * st["bucket_columns"][b]
         except Exception:
             traffic = None
     roofline = {"bound": "fp32", "achieved": achieved, "peak": peak32, "unit": "TFLOP/s",
                 "frac": (achieved / peak32) if achieved else None, "traffic": traffic,
-                "kernel": ["warp_solve_kernel", "fixed_solve_kernel (first launch)",
-                           "fixed_solve_kernel (large arena)", "cta_solve_kernel (fallback)"][b],
+                "kernel": kernel,
                 "kernel_ms": kms, "flops_per_launch": st["bucket_flops"][b],
                 "peak_source": "measured FP32 FMA probe (mspai_measure_fma_peak)"}
 
