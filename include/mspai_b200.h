@@ -116,9 +116,14 @@ typedef struct {
                          and B have the structure of the last setup that kept
                          its factors (keep_factors, same precision), every
                          column of the fixed-pattern solver starts from its
-                         previous solution and R and takes at most this many
-                         FP64 refinement steps against the new values; a
-                         column that does not converge is factored again.
+                         previous solution.  Columns with a diagonally
+                         dominant normal matrix iterate on it to rounding
+                         level without R (from zero when the values have
+                         changed too much): this bound does not count there,
+                         and their kept R stays that of the older values.
+                         The others take at most this many FP64 refinement
+                         steps with their kept R against the new values; one
+                         that does not converge is factored again.
                          The reference's update path keeps each column's QR
                          across setups (src/Spai_Update.imp:45-325); 0
                          recomputes every column (0)                       */
@@ -142,7 +147,8 @@ typedef struct {
     int64_t kernel_launches;  /* kernels this library launched in the setup  */
     double bucket_flops[4];   /* algorithmic (folded) flops per bucket kernel */
     int64_t reused_columns;   /* columns that took an identical column's solution (-cs/-ch) */
-    int64_t factor_reuse_columns; /* columns that converged from their kept factor */
+    int64_t factor_reuse_columns; /* columns of a re-setup that converged from their
+                                 previous solution (reuse_factors)          */
 } mspai_stats;
 
 typedef struct mspai_handle mspai_handle;
@@ -274,9 +280,11 @@ int mspai_solver_columns(mspai_handle* h, int64_t* counts);
  * nonzeros of B; *loss receives L.  gbar_values (nnz(M) values in M's order)
  * may be NULL.  All value arrays live where `mem` says.  The residual term
  * needs no solve (M is stationary); the gbar term needs
- * lambda_k = R_k^-1 R_k^-T gbar_k: from the R that the setup kept
- * (keep_factors; refined in FP64 when R is FP32), else from R recomputed in
- * FP64.  Q is never stored.  Not in the reference.
+ * lambda_k = (C_k^T C_k)^-1 gbar_k.  Columns with a diagonally dominant normal
+ * matrix iterate on it without a factor; the others take R_k^-1 R_k^-T from the
+ * R that the setup kept (keep_factors; refined in FP64 against C, since R may be
+ * FP32 or of the values before a re-setup), else, or when that does not converge,
+ * from R recomputed in FP64.  Q is never stored.  Not in the reference.
  */
 int mspai_adjoint(mspai_handle* h, const mspai_csc* C, const mspai_csc* B,
                   const double* gbar_values, double* dC_values, double* dB_values,

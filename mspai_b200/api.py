@@ -50,7 +50,8 @@ class Options:
     col_begin: int = 0         # solve only columns [col_begin, col_end) (0, 0: all)
     col_end: int = 0
     keep_factors: bool = False  # keep every column's R (adjoint's gbar term, re-setups)
-    reuse_factors: int = 0      # > 0: re-setup from the kept factors, at most this many steps
+    reuse_factors: int = 0      # > 0: re-setup from the previous solution and kept factors
+                                # (at most this many steps with a kept factor)
 
     def to_c(self) -> mspai_params:
         p = mspai_params()
