@@ -415,6 +415,10 @@ __device__ bool hub_solve(CgShared& sh, int& parity, const SharedEntries& g, con
             if (lane < nh)
                 L[lane * kHubLd + j] = Fixed<T>::value(schur[lane * kHubLd + j]);
         __syncwarp();
+        // FP64 without refinement: beyond a condition of 2^13 the first correction
+        // does not reach 2^-44 (1 is the largest pivot of the scaled matrix), so the
+        // column is refused here and not after two corrections
+        const T least = pb.refine > 0 ? T(0) : T(0x1p-13);
         bool bad = false;
 #pragma unroll 1
         for (int j = 0; j < nh; j++) {
@@ -425,7 +429,7 @@ __device__ bool hub_solve(CgShared& sh, int& parity, const SharedEntries& g, con
                     s -= L[lane * kHubLd + k] * L[j * kHubLd + k];
             }
             const T piv = __shfl_sync(kNone, s, j);
-            bad = bad || !(piv > T(0));
+            bad = bad || !(piv > least);
             const T iv = T(1) / tsqrt<T>(bad ? T(1) : piv);
             if (lane == j)
                 inv = iv;

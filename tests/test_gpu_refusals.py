@@ -294,3 +294,29 @@ def test_small_block_columns_beside_large_ones_in_fp64(h):
     small = np.repeat(np.diff(P.indptr) == 6, bs)
     assert h.solver_columns()["general"] >= 54
     assert np.allclose(res[small], np.asarray(o.res).ravel()[small], rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("near,refused", [(0.0, False), (3e-2, True)])
+def test_small_fp64_columns_by_condition(h, near, refused):
+    """FP64 without refinement: elimination takes well-conditioned columns of 20
+    unknowns and leaves those with two nearly parallel columns to the QR.  The
+    residual norm does not change to first order in the solution's error, so that
+    rounding leaves it within 1e-12 of the smallest one at condition 1e3."""
+    n = 300
+    A = matrix(n, 4, 6.0, seed=13)
+    if near:
+        D = A.toarray()
+        noise = np.random.default_rng(14).standard_normal(D[:, 0::2].shape)
+        D[:, 1::2] = D[:, 0::2] * (1.0 + near * noise)
+        A = sp.csc_matrix(D)
+        A.sort_indices()
+    P = pattern(n, (20,), seed=15).tolil()
+    P[:2] = 1.0
+    P = sp.csc_matrix(P)
+    P.sort_indices()
+    h.setup(A, P, options=mb.Options(ns=0, prec="fp64"))
+    c = h.solver_columns()
+    assert c["sparse_small"] == n and c["fixed"] == (n if refused else 0)
+    res, _, status = h.column_info()
+    assert np.all(status == 0)
+    assert np.allclose(res, O.spai_scalar(A, P, ns=0).res, rtol=1e-12, atol=1e-12)
