@@ -104,9 +104,8 @@ __device__ Fit block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Probl
     const int most_rows = min(E, room / (8 + 8 * bs + 4 * static_cast<int>(sizeof(T))));
     if (most_rows < 1)
         return Fit::kLarger;
-    const bool limited = most_rows < E;
-    const int hs = next_pow2(max(64, limited ? min(E + E / 2, most_rows + most_rows / 4 + NT)
-                                             : E + E / 2));
+    const int hs = next_pow2(max(
+        64, most_rows < E ? min(E + E / 2, most_rows + most_rows / 4 + NT) : E + E / 2));
     const int hbits = 31 - __clz(hs);
     int32_t* key = a.high<int32_t>(hs);
     int32_t* first = a.high<int32_t>(hs);
@@ -122,7 +121,7 @@ __device__ Fit block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Probl
     const volatile int* rows = &fs.mcount;
     for (int jj = tid / 8; jj < n; jj += NT / 8) {
         const int o = off[jj], len = off[jj + 1] - o;
-        for (int q = tid & 7; q < len && (!limited || *rows <= most_rows); q += 8) {
+        for (int q = tid & 7; q < len && *rows <= most_rows; q += 8) {
             const int row = __ldg(pb.cidx + cb[jj] + q);
             uint32_t s = (static_cast<uint32_t>(row) * 2654435761u) >> (32 - hbits);
             int old = atomicCAS(&key[s], -1, row);
@@ -130,14 +129,14 @@ __device__ Fit block_column(const CtaGroup<NT>& g, FixShared<T>& fs, const Probl
                 s = (s + 1) & (hs - 1);
                 old = atomicCAS(&key[s], -1, row);
             }
-            if (limited && old == -1)
+            if (old == -1)
                 atomicAdd(&fs.mcount, 1);
             atomicMin(&first[s], o + q);
             R[o + q] = static_cast<uint16_t>(s);
         }
     }
     g.sync();
-    if (limited && fs.mcount > most_rows)
+    if (fs.mcount > most_rows)
         return Fit::kLarger;
     for (int e = tid; e < E; e += NT)
         flag[e] = first[R[e]] == e ? 1 : 0;
@@ -614,7 +613,8 @@ __global__ void __launch_bounds__(128)
     }
 }
 
-template <class T, int NT, int MINB>
+// kLast: no larger arena follows.
+template <class T, int NT, int MINB, bool kLast>
 __global__ void __launch_bounds__(NT, MINB)
     block_solve_kernel(Problem pb, Output out, const int32_t* __restrict__ list,
                        const int32_t* __restrict__ count_dev, int count_host,
@@ -637,18 +637,20 @@ __global__ void __launch_bounds__(NT, MINB)
         const int kb = list[t];
         const Fit fit = block_column<T, NT>(g, fs, pb, out, kb, smem, arena_bytes);
         if (fit != Fit::kYes && threadIdx.x == 0) {
-            const WorkList& to = fit == Fit::kLarger ? larger : left;
-            to.list[atomicAdd(to.count, 1)] = kb;
+            if (!kLast && fit == Fit::kLarger)
+                larger.list[atomicAdd(larger.count, 1)] = kb;
+            else
+                left.list[atomicAdd(left.count, 1)] = kb;
         }
     }
 }
 
-template <class T, int NT, int MINB>
+template <class T, int NT, int MINB, bool kLast>
 cudaError_t launch_block_t(int arena, const Problem& pb, const Output& out, const int32_t* list,
                            const int32_t* count_dev, int count, int32_t* counter,
                            const WorkList& larger, const WorkList& left, cudaStream_t st)
 {
-    auto kern = block_solve_kernel<T, NT, MINB>;
+    auto kern = block_solve_kernel<T, NT, MINB, kLast>;
     cudaError_t e =
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, arena);
     if (e != cudaSuccess)
@@ -679,14 +681,14 @@ cudaError_t launch_block_solve(int elem_bytes, const Problem& pb, const Output& 
     block_small_kernel<<<blocks, 128, 0, st>>>(pb, out, list, count, wide, left);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess)
-        e = launch_block_t<double, 64, 8>(15 * 1024, pb, out, wide.list, wide.count, count,
+        e = launch_block_t<double, 64, 8, false>(15 * 1024, pb, out, wide.list, wide.count, count,
                                            counts + 3, large, left, st);
     if (e != cudaSuccess)
         return e;
     if (elem_bytes == 4)
-        return launch_block_t<float, 256, 2>(107 * 1024, pb, out, large.list, large.count, count,
+        return launch_block_t<float, 256, 2, true>(107 * 1024, pb, out, large.list, large.count, count,
                                              counts + 4, left, left, st);
-    return launch_block_t<double, 256, 1>(212 * 1024, pb, out, large.list, large.count, count,
+    return launch_block_t<double, 256, 1, true>(212 * 1024, pb, out, large.list, large.count, count,
                                           counts + 4, left, left, st);
 }
 
