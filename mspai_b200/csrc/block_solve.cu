@@ -25,8 +25,9 @@
 //   Bound: latency of the blocked Cholesky and of the triangular solves at two
 //   CTAs of 256 threads per SM (mixed), one (FP64).  8,000 block columns of a
 //   20^3 27-point stencil with 3 x 3 blocks: 36.9 ms in the general solver, 12.7 ms
-//   here with a walk over C's values per right-hand side, 6.7 ms with one for all; 64,000 of the block diagonal (3 unknowns, 246 entries, eight lanes
-//   each; CTAs of 64 threads took 2.7): 3.6 ms there, 1.7 ms here.
+//   here with a walk over C's values per right-hand side, 6.8 ms with one for all;
+//   64,000 of the block diagonal (3 unknowns, 246 entries, eight lanes each; CTAs of
+//   64 threads took 2.7): 3.6 ms there, 1.7 ms here.
 #include "fixed_solve.cuh"
 #include "spai_kernels.h"
 
