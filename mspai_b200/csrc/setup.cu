@@ -29,9 +29,9 @@ using mspai::Problem;
 constexpr int kBuckets = 3;    // size buckets of the planning kernel
 constexpr int kKernels = 4;    // solver launches per setup (timed separately)
 constexpr int kLists = 4;      // work lists: buckets + the overflow lists
-constexpr int kMoreLists = 5;  // ... two between the sparse solvers' launches, their small
+constexpr int kMoreLists = 6;  // ... two between the sparse solvers' launches, their small
                                // columns, the small QR's columns, its tall ones and, after
-                               // these, the sparse solvers' refused columns
+                               // these, the sparse solvers' refused columns, the small QR's
 // Arena of the fixed-pattern solver's second launch (one CTA per SM): the
 // largest dynamic shared memory a CTA may have beside the solver's static part.
 constexpr int kFixedArenaLarge = 212 * 1024;
@@ -146,6 +146,7 @@ struct mspai_handle {
     int64_t list_len[kLists] = {};   // columns listed per work list in the last setup
     int64_t tiny_len = 0;            // ... in the sparse solvers' list of small columns
     int64_t small_len = 0;           // ... and in the small QR's
+    int32_t* refused_any = nullptr;  // pinned: the small QR has refused columns
     // columns handed to each solver in the last setup: a number, plus the device
     // counter handed_at (-1: none), which stays until the next setup
     int64_t handed[MSPAI_SOLVERS] = {};
@@ -290,6 +291,8 @@ void mspai_free(mspai_handle* h)
                       &h->rglob, &h->aloss, &h->acnt, &h->alists};
     for (DevBuf* b : bufs)
         b->release();
+    if (h->refused_any)
+        cudaFreeHost(h->refused_any);
     if (h->ev0)
         cudaEventDestroy(h->ev0);
     if (h->ev1)
@@ -759,12 +762,18 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
     if (nsmall > 0) {
         int32_t* lists = h->lists.as<int32_t>();
         int32_t* rc = dcnt + 36;
-        CUDA_TRY(h, cudaMemsetAsync(rc, 0, 2 * sizeof(int32_t), st));
+        if (!h->refused_any)
+            CUDA_TRY(h, cudaHostAlloc(reinterpret_cast<void**>(&h->refused_any), sizeof(int32_t),
+                                      cudaHostAllocDefault));
+        *h->refused_any = 0;  // the stream is idle: no kernel of this handle writes it now
+        CUDA_TRY(h, cudaMemsetAsync(rc, 0, 3 * sizeof(int32_t), st));
         CUDA_TRY(h, cudaEventRecord(h->evb[0], st));
         h->launches += 2;
         CUDA_TRY(h, mspai::launch_small_qr(
                         pb, out, lists + static_cast<size_t>(kLists + 3) * nprob, nsmall,
-                        lists + static_cast<size_t>(kLists + 4) * nprob, rc, st));
+                        lists + static_cast<size_t>(kLists + 4) * nprob, rc,
+                        {lists + static_cast<size_t>(kLists + 5) * nprob, rc + 2}, h->refused_any,
+                        st));
         CUDA_TRY(h, cudaEventRecord(h->evb[1], st));
         timed[0] = true;
         h->stats.bucket_columns[0] = nsmall;
@@ -1058,6 +1067,33 @@ int mspai_setup(mspai_handle* h, const mspai_csc* C, const mspai_csc* C_rows, co
     }
     CUDA_TRY(h, cudaEventRecord(h->ev1, st));
     CUDA_TRY(h, cudaStreamSynchronize(st));
+    if (nsmall > 0 && *static_cast<volatile int32_t*>(h->refused_any)) {
+        // singular or overflowing columns of the small QR: the warp solver
+        int32_t nref = 0;
+        CUDA_TRY(h, cudaMemcpy(&nref, dcnt + 38, sizeof(int32_t), cudaMemcpyDeviceToHost));
+        Caps cap{};
+        cap.emax = mspai::kSmallE;
+        cap.nmax = mspai::kSmallN;
+        cap.lsort = mspai::next_pow2(cap.emax);
+        cap.mwmax = cap.emax / 2 + cap.nmax;
+        cap.nrhs = 1;
+        Problem pbs = pb;
+        pbs.refine = 0;  // FP64, as every bucket of so few unknowns
+        int grid = 0;
+        CUDA_TRY(h, cudaMemsetAsync(dcnt + 12, 0, sizeof(int32_t), st));
+        h->launches++;
+        h->handed[MSPAI_SOLVER_WARP] += nref;
+        CUDA_TRY(h, mspai::launch_warp_solve(
+                        8, pbs, cap, out, h->lists.as<int32_t>() +
+                                              static_cast<size_t>(kLists + 5) * nprob,
+                        nref, dcnt + 12, st, &grid));
+        if (reuse) {
+            h->launches++;
+            CUDA_TRY(h, mspai::launch_reuse_copy(drep, nprob, bs, out, st));
+        }
+        CUDA_TRY(h, cudaEventRecord(h->ev1, st));
+        CUDA_TRY(h, cudaStreamSynchronize(st));
+    }
     CUDA_TRY(h, cudaGetLastError());
     float ms = 0.f;
     cudaEventElapsedTime(&ms, h->ev0, h->ev1);

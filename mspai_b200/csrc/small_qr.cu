@@ -11,7 +11,9 @@
 // in shared memory in row order.  Lane l then takes rows l, l + 8, ... into
 // registers and the group factors them by Householder reflections (dlarfg:
 // beta = -sign(alpha) ||(alpha, x)||, tau = 0 for x = 0) with three-step sums.
-// The residual is formed in FP64 from the matrix in shared memory.
+// The residual is formed in FP64 from the matrix in shared memory.  A column whose
+// solution is not finite (a zero on R's diagonal, an overflow) is left to the general
+// warp solver: on dependent columns the two meet exact zeros in different places.
 //   Bound: FP64 latency (a square root and a reciprocal per reflection) at 16
 //   warps per SM (128 registers, 38 KB of shared memory a CTA of four warps; columns
 //   of 33 to 64 rows: 8).  Anisotropic 1024^2 with two probing rows: 13.6 ms in the
@@ -42,7 +44,8 @@ template <int R>
 __global__ void __launch_bounds__(kSmallThreads)
     small_qr_kernel(Problem pb, Output out, const int32_t* __restrict__ list,
                     const int32_t* __restrict__ count_dev, int count_host,
-                    int32_t* __restrict__ rest, int32_t* __restrict__ rest_count)
+                    int32_t* __restrict__ rest, int32_t* __restrict__ rest_count,
+                    WorkList refused, int32_t* __restrict__ refused_any)
 {
     constexpr int M = 8 * R;
     extern __shared__ __align__(16) char smem[];
@@ -137,7 +140,6 @@ __global__ void __launch_bounds__(kSmallThreads)
         const int nmax = __reduce_max_sync(kAll, n), mmax = __reduce_max_sync(kAll, min(m, M));
         // ---- Householder QR, the reflectors unscaled: v = scale x
         double rinv = 0.0;  // lane k: 1 / R(k, k)
-        bool zero = false;  // a zero diagonal of R
 #pragma unroll
         for (int k = 0; k < 8; k++) {
             if (k >= nmax)
@@ -159,11 +161,8 @@ __global__ void __launch_bounds__(kSmallThreads)
             else {
                 ib = 1.0 / alpha;
             }
-            if (k < n) {
-                zero = zero || beta == 0.0;
-                if (l8 == k)
-                    rinv = ib;
-            }
+            if (k < n && l8 == k)
+                rinv = ib;
             // v^T of the later columns and of the right-hand side
             double d[9];
 #pragma unroll
@@ -199,7 +198,7 @@ __global__ void __launch_bounds__(kSmallThreads)
                 }
             }
         }
-        // ---- back substitution; R singular: x = (Q^T b)(0:n), as dtrtrs leaves B
+        // ---- back substitution; x is not finite when R has a zero on its diagonal
         double x = b[0];
         double xs[8];
 #pragma unroll
@@ -207,11 +206,11 @@ __global__ void __launch_bounds__(kSmallThreads)
             xs[k] = 0.0;
             if (k >= nmax)
                 continue;
-            if (!zero && l8 == k && k < n)
+            if (l8 == k && k < n)
                 x *= rinv;
             const double xk = __shfl_sync(kAll, x, k, 8);
             xs[k] = k < n ? xk : 0.0;
-            if (!zero && l8 < k && k < n)
+            if (l8 < k && k < n)
                 x -= a[0][k] * xk;
         }
         // ---- FP64 residual from the matrix
@@ -230,7 +229,14 @@ __global__ void __launch_bounds__(kSmallThreads)
         r2 = group_sum(r2);
         const uint32_t odd = __ballot_sync(kAll, l8 < n && !isfinite(x));
         __syncwarp();
-        if (live) {
+        const bool bad = ((odd >> (8 * grp)) & 0xffu) != 0 || !isfinite(r2);
+        if (live && bad) {
+            if (l8 == 0) {
+                refused.list[atomicAdd(refused.count, 1)] = col;
+                *refused_any = 1;
+            }
+        }
+        else if (live) {
             if (l8 < n)
                 out.oval[p0 + l8] = x;
             if (l8 == 0) {
@@ -244,8 +250,7 @@ __global__ void __launch_bounds__(kSmallThreads)
                 out.olen[col] = n;
                 out.res[col] = res;
                 out.steps[col] = 1;
-                const bool bad = ((odd >> (8 * grp)) & 0xffu) != 0 || !isfinite(res);
-                out.status[col] = zero ? 1 : (bad ? 2 : 0);
+                out.status[col] = 0;
             }
         }
     }
@@ -254,7 +259,8 @@ __global__ void __launch_bounds__(kSmallThreads)
 template <int R>
 cudaError_t launch_small_t(const Problem& pb, const Output& out, const int32_t* list,
                            const int32_t* count_dev, int count_host, int32_t* rest,
-                           int32_t* rest_count, cudaStream_t st)
+                           int32_t* rest_count, const WorkList& refused, int32_t* refused_any,
+                           cudaStream_t st)
 {
     auto kern = small_qr_kernel<R>;
     const int bytes = (kSmallThreads / 8) * 8 * R *
@@ -271,20 +277,23 @@ cudaError_t launch_small_t(const Problem& pb, const Output& out, const int32_t* 
     const int per_cta = kSmallThreads / 8;
     const int grid = std::max(1, std::min(per_sm * num_sms(), (count_host + per_cta - 1) / per_cta));
     kern<<<grid, kSmallThreads, bytes, st>>>(pb, out, list, count_dev, count_host, rest,
-                                             rest_count);
+                                             rest_count, refused, refused_any);
     return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_small_qr(const Problem& pb, const Output& out, const int32_t* list, int count,
-                            int32_t* rest, int32_t* rest_count, cudaStream_t st)
+                            int32_t* rest, int32_t* rest_count, const WorkList& refused,
+                            int32_t* refused_any, cudaStream_t st)
 {
-    cudaError_t e = launch_small_t<4>(pb, out, list, nullptr, count, rest, rest_count, st);
+    cudaError_t e = launch_small_t<4>(pb, out, list, nullptr, count, rest, rest_count, refused,
+                                      refused_any, st);
     if (e != cudaSuccess)
         return e;
     // the columns of 33 to 64 rows (at most 64 entries: none is left)
-    return launch_small_t<8>(pb, out, rest, rest_count, count, rest, rest_count + 1, st);
+    return launch_small_t<8>(pb, out, rest, rest_count, count, rest, rest_count + 1, refused,
+                             refused_any, st);
 }
 
 }  // namespace mspai

@@ -103,18 +103,20 @@ cudaError_t launch_fixed_solve(int elem_bytes, int arena_bytes, const Problem& p
                                int count_host, int32_t* counter, int32_t* ovf_list,
                                int32_t* ovf_count, void* rglob, int64_t rglob_elems, int max_ctas,
                                cudaStream_t st, int* grid_out);
-// Columns of at most eight unknowns and 64 entries of C(:, J) (small_qr.cu):
-// FP64 Householder QR, eight lanes per column.  rest (count entries) and
-// rest_count[2] (zero) are scratch.
-constexpr int kSmallN = 8;
-constexpr int kSmallE = 64;
-cudaError_t launch_small_qr(const Problem& pb, const Output& out, const int32_t* list, int count,
-                            int32_t* rest, int32_t* rest_count, cudaStream_t st);
 // A work list in device memory that columns are appended to.
 struct WorkList {
     int32_t* list;
     int32_t* count;
 };
+// Columns of at most eight unknowns and 64 entries of C(:, J) (small_qr.cu):
+// FP64 Householder QR, eight lanes per column.  rest (count entries) and
+// rest_count[2] (zero) are scratch.  refused: columns without a finite solution (nothing
+// of them is written); *refused_any (host memory) is set when there are any.
+constexpr int kSmallN = 8;
+constexpr int kSmallE = 64;
+cudaError_t launch_small_qr(const Problem& pb, const Output& out, const int32_t* list, int count,
+                            int32_t* rest, int32_t* rest_count, const WorkList& refused,
+                            int32_t* refused_any, cudaStream_t st);
 // Solvers on the sparse normal equations (fixed_cg.cu), a CTA per column in
 // slot_bytes of shared memory.  The columns that do not fit the slot go to
 // `larger`; to `refused` those that no slot up to `widest` bytes would take.

@@ -320,3 +320,46 @@ def test_small_fp64_columns_by_condition(h, near, refused):
     res, _, status = h.column_info()
     assert np.all(status == 0)
     assert np.allclose(res, O.spai_scalar(A, P, ns=0).res, rtol=1e-12, atol=1e-12)
+
+
+@pytest.mark.parametrize("sizes", [(4,), (7, 3)])
+@pytest.mark.parametrize("cs", [0, 100])
+def test_small_dependent_columns(h, sizes, cs):
+    """Two equal columns in every J of at most eight: rounding decides whether a QR
+    meets an exact zero.  What the small QR does not solve is the warp solver's,
+    with its values and its status bit for bit (a setup that keeps the factors
+    uses the warp solver alone)."""
+    n = 300
+    D = matrix(n, 6, 3.0, seed=16).toarray()
+    D[:, 1::3] = D[:, 0::3]
+    D[:, 2] = 0.0
+    A = sp.csc_matrix(D)
+    # an explicit zero column: a zero on the diagonal whatever the rounding
+    A = sp.csc_matrix(A + sp.csc_matrix(([1.0], ([5], [2])), shape=A.shape))
+    A.data[A.indptr[2]:A.indptr[3]] = 0.0
+    P = pattern(n, sizes, seed=17).toarray()
+    both = np.maximum(P[0::3], P[1::3])
+    P[0::3], P[1::3] = both, both
+    P[2, 30:40] = 1.0
+    P = sp.csc_matrix(P)
+    P.sort_indices()
+    assert P.getnnz(axis=0).max() <= 15
+    small = P.getnnz(axis=0) <= 8
+    h.setup(A, P, options=mb.Options(ns=0, prec="fp64", cs=cs))
+    M, c = h.result(), h.solver_columns()
+    res, steps, status = h.column_info()
+    assert c["small_qr"] > 0 and 0 < c["warp"]
+    ref = mb.Handle(0)
+    ref.setup(A, P, options=mb.Options(ns=0, prec="fp64", keep_factors=True))
+    N = ref.result()
+    rres, _, rstatus = ref.column_info()
+    ref.close()
+    assert np.array_equal(status[small], rstatus[small])
+    zero = np.flatnonzero(small & (P[2].toarray().ravel() != 0))
+    assert zero.size > 0 and np.all(status[zero] == 1)
+    same = 0
+    for k in np.flatnonzero(small):
+        a, b = M.indptr[k], M.indptr[k + 1]
+        if np.array_equal(M.data[a:b], N.data[a:b]) and res[k] == rres[k]:
+            same += 1
+    assert same >= (c["warp"] if cs == 0 else 1) - np.count_nonzero(~small)
